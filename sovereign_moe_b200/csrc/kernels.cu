@@ -7,6 +7,7 @@
 #include <map>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "common.cuh"
 
@@ -491,70 +492,176 @@ __global__ void pdhg_accum_kernel(int n, double* acc, const double* inc, double*
 
 enum { RED_DOT = 0, RED_SQ = 1, RED_ABSMAX = 2 };
 
-__device__ __forceinline__ double red_combine(double a, double b, int op) {
-  return op == RED_ABSMAX ? fmax(a, b) : a + b;
+template <int OP>
+__device__ __forceinline__ double red_combine(double a, double b) {
+  return OP == RED_ABSMAX ? fmax(a, b) : a + b;
 }
 
-// Block-level partial of a reduction over [0, n) with a grid-stride loop of
-// fixed shape: partials[blockIdx.x].  Deterministic for a given grid.
-__global__ void __launch_bounds__(kT) reduce_partial_kernel(long long n, const double* a,
-                                                            const double* b, int op,
-                                                            double* partials) {
-  __shared__ double sh[kT / 32];
-  double acc = 0.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double v = a[i];
-    const double t = op == RED_DOT ? v * b[i] : (op == RED_SQ ? v * v : fabs(v));
-    acc = red_combine(acc, t, op);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc = red_combine(acc, __shfl_down_sync(kAll, acc, off), op);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (kT / 32) ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = red_combine(v, __shfl_down_sync(kAll, v, off), op);
-    if (threadIdx.x == 0) partials[blockIdx.x] = v;
-  }
+// The term of one element added to a running sum (a fused multiply-add: one
+// rounding per element).
+template <int OP>
+__device__ __forceinline__ double red_add(double acc, double a, double b) {
+  if (OP == RED_DOT) return fma(a, b, acc);
+  if (OP == RED_SQ) return fma(a, a, acc);
+  return fmax(acc, fabs(a));
 }
 
-__global__ void __launch_bounds__(kT) reduce_final_kernel(int nparts, const double* partials,
-                                                          int op, double* out) {
-  __shared__ double sh[kT / 32];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc = red_combine(acc, partials[i], op);
+// Sum over a block of kT threads: a fixed shuffle tree in each warp, then the
+// warp sums in a tree; the result is thread 0's.
+template <int OP>
+__device__ __forceinline__ double red_block(double acc, double* sh) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc = red_combine(acc, __shfl_down_sync(kAll, acc, off), op);
+  for (int off = 16; off > 0; off >>= 1) acc = red_combine<OP>(acc, __shfl_down_sync(kAll, acc, off));
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
+  double v = threadIdx.x < (kT / 32) ? sh[threadIdx.x] : 0.0;
   if (threadIdx.x < 32) {
-    double v = threadIdx.x < (kT / 32) ? sh[threadIdx.x] : 0.0;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = red_combine(v, __shfl_down_sync(kAll, v, off), op);
-    if (threadIdx.x == 0) *out = v;
+    for (int off = 16; off > 0; off >>= 1) v = red_combine<OP>(v, __shfl_down_sync(kAll, v, off));
   }
+  return v;
 }
 
 constexpr int kRedBlocks = 592;   // 4 x 148 SMs: fixed, so results do not depend on the device
+
+// A whole reduction over [0, n) in one launch.  Element i goes to thread
+// i mod (kRedBlocks kT), as a grid of kRedBlocks blocks strides over the
+// vector; the launch holds only the blocks that have elements (the others'
+// partials would be zeros, which change no sum of squares, products or
+// maximum of magnitudes).  The last block to finish adds the block partials
+// in a fixed order and writes the result to pinned host memory, so a call is
+// one launch and one synchronisation.  Deterministic: the order depends on n
+// alone.
+template <int OP>
+__global__ void __launch_bounds__(kT) reduce_kernel(long long n, const double* __restrict__ a,
+                                                    const double* __restrict__ b,
+                                                    double* __restrict__ partials,
+                                                    unsigned* __restrict__ done,
+                                                    double* __restrict__ out) {
+  __shared__ double sh[kT / 32];
+  __shared__ bool last;
+  constexpr long long kStride = (long long)kRedBlocks * kT;
+  constexpr int kU = 4;             // elements in flight per thread, added in order
+  double acc = 0.0;
+  long long i = (long long)blockIdx.x * kT + threadIdx.x;
+  for (; i + (kU - 1) * kStride < n; i += kU * kStride) {
+    double va[kU], vb[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      va[u] = a[i + u * kStride];
+      vb[u] = OP == RED_DOT ? b[i + u * kStride] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) acc = red_add<OP>(acc, va[u], vb[u]);
+  }
+  for (; i < n; i += kStride) acc = red_add<OP>(acc, a[i], OP == RED_DOT ? b[i] : 0.0);
+  acc = red_block<OP>(acc, sh);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = acc;
+    __threadfence();                // the partial is visible before the count
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();                  // every other block's partial after its count
+  double f = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += kT) f = red_combine<OP>(f, __ldcg(partials + k));
+  f = red_block<OP>(f, sh);
+  if (threadIdx.x == 0) {
+    *out = f;
+    *done = 0;                      // ready for the slot's next call
+  }
+}
+
+// What one reduction in flight needs: block partials and a counter on the
+// device, a pinned host word for the result.  A call takes a slot for its
+// duration (it returns after its stream has been waited for), so calls on
+// any threads and streams never share one.  At most kRedSlots per device are
+// kept between calls, 5 KB each; a call that finds all of them taken makes a
+// slot of its own and releases it.  (Scratch from the stream-ordered pool, as
+// before, cost about 430 us per call: the pool returns its memory at every
+// synchronisation, and every reduction synchronises.)
+struct RedSlot {
+  double* partials = nullptr;       // [kRedBlocks]
+  unsigned* done = nullptr;
+  double* out = nullptr;            // pinned, mapped
+  double* out_dev = nullptr;        // its device address
+};
+constexpr int kRedSlots = 16;
+std::mutex red_mu;
+struct RedPool {
+  std::vector<RedSlot> free;
+  int kept = 0;                     // slots that go back to the pool: free or in use
+};
+std::map<int, RedPool> red_pools;   // by device
+
+void red_free(RedSlot& s) {
+  if (s.partials) cudaFree(s.partials);
+  if (s.out) cudaFreeHost(s.out);
+  s = RedSlot{};
+}
+
+cudaError_t red_make(RedSlot& s, cudaStream_t st) {
+  // allocating is allowed while another thread captures a stream
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  cudaError_t e = cudaMalloc((void**)&s.partials, sizeof(double) * (kRedBlocks + 1));
+  if (e == cudaSuccess) {
+    s.done = reinterpret_cast<unsigned*>(s.partials + kRedBlocks);
+    e = cudaHostAlloc((void**)&s.out, sizeof(double), cudaHostAllocMapped);
+  }
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&s.out_dev, s.out, 0);
+  // zero before the first launch on the slot, which is on this stream; later
+  // ones follow a call that has waited for its stream
+  if (e == cudaSuccess) e = cudaMemsetAsync(s.done, 0, sizeof(unsigned), st);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) red_free(s);
+  return e;
+}
 
 int reduce(long long n, const double* a, const double* b, int op, double* out, cudaStream_t st) {
   if (!out) return fail(PDLP_ERR_ARG, "out is NULL");
   if (n < 0) return fail(PDLP_ERR_ARG, "n must be >= 0");
   if (n == 0) { *out = 0.0; return PDLP_OK; }
   if (!a || (op == RED_DOT && !b)) return fail(PDLP_ERR_ARG, "NULL pointer");
-  // scratch: block partials and the result, from the stream-ordered pool
-  double* scratch = nullptr;
-  PDLP_CUDA(cudaMallocAsync((void**)&scratch, sizeof(double) * (kRedBlocks + 1), st));
-  reduce_partial_kernel<<<kRedBlocks, kT, 0, st>>>(n, a, b, op, scratch);
-  reduce_final_kernel<<<1, kT, 0, st>>>(kRedBlocks, scratch, op, scratch + kRedBlocks);
-  count_launches(2);
-  cudaError_t e = cudaGetLastError();
-  double h = 0.0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, scratch + kRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, st);
-  cudaFreeAsync(scratch, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  int dev = 0;
+  PDLP_CUDA(cudaGetDevice(&dev));
+  RedSlot s;
+  bool kept = false;                // the slot goes back to the pool
+  {
+    std::lock_guard<std::mutex> lock(red_mu);
+    RedPool& p = red_pools[dev];
+    if (!p.free.empty()) {
+      s = p.free.back();
+      p.free.pop_back();
+      kept = true;
+    } else if (p.kept < kRedSlots) {
+      ++p.kept;
+      kept = true;
+    }
+  }
+  cudaError_t e = s.partials ? cudaSuccess : red_make(s, st);
+  if (e == cudaSuccess) {
+    const int g = (int)std::min<long long>(kRedBlocks, (n + kT - 1) / kT);
+    if (op == RED_DOT) reduce_kernel<RED_DOT><<<g, kT, 0, st>>>(n, a, b, s.partials, s.done, s.out_dev);
+    else if (op == RED_SQ) reduce_kernel<RED_SQ><<<g, kT, 0, st>>>(n, a, b, s.partials, s.done, s.out_dev);
+    else reduce_kernel<RED_ABSMAX><<<g, kT, 0, st>>>(n, a, b, s.partials, s.done, s.out_dev);
+    count_launches(1);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  const double h = e == cudaSuccess ? *s.out : 0.0;
+  if (e != cudaSuccess || !kept) {
+    // a failed call may have left the counter between two values
+    red_free(s);
+    if (kept) {
+      std::lock_guard<std::mutex> lock(red_mu);
+      --red_pools[dev].kept;
+    }
+  } else {
+    std::lock_guard<std::mutex> lock(red_mu);
+    red_pools[dev].free.push_back(s);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "reduction");
   *out = op == RED_SQ ? sqrt(h) : h;
   return PDLP_OK;
@@ -596,6 +703,17 @@ __global__ void __launch_bounds__(kT) dot_chunk_kernel(long long n, const double
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(kAll, v, off);
     if (threadIdx.x == 0) partials[blockIdx.x] = v;
   }
+}
+
+// *out = the sum of the chunk sums, by one block in a fixed order.
+__global__ void __launch_bounds__(kT) dot_final_kernel(int nparts,
+                                                       const double* __restrict__ partials,
+                                                       double* __restrict__ out) {
+  __shared__ double sh[kT / 32];
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < nparts; i += kT) acc += partials[i];
+  acc = red_block<RED_DOT>(acc, sh);
+  if (threadIdx.x == 0) *out = acc;
 }
 
 // Device address of noalloc_scratch, looked up once per device ordinal (with
@@ -754,7 +872,7 @@ int pdlp_dot_noalloc(int64_t n, const double* a, const double* b, double* out, v
   // in the scratch has to start at zero
   const int chunks = (int)((n + kNaChunk - 1) / kNaChunk);
   dot_chunk_kernel<<<chunks, kT, 0, st>>>(n, a, b, scratch);
-  reduce_final_kernel<<<1, kT, 0, st>>>(chunks, scratch, RED_DOT, scratch + kNaMaxChunks);
+  dot_final_kernel<<<1, kT, 0, st>>>(chunks, scratch, scratch + kNaMaxChunks);
   count_launches(2);
   cudaError_t e = cudaGetLastError();
   double h = 0.0;
