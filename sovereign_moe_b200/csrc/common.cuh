@@ -65,6 +65,19 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
+// Programmatic dependent launch.  grid_dep_wait returns once the kernel
+// before this one in the stream has completed and its writes are visible (at
+// once when there is none); grid_dep_release lets the next kernel in the
+// stream, if it was launched as a programmatic dependent, start its CTAs as
+// this kernel's CTAs leave the SMs.
+__device__ __forceinline__ void grid_dep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ void grid_dep_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ long long global_ns() {
   long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -24,7 +24,8 @@ int grid_1d(long long n, int per = kT) {
 
 // y = A x in two launches, with a fixed summation order.
 //
-// spmv_rows32_kernel: one warp per block of 32 consecutive rows.  Rows with
+// spmv_rows_kernel: one warp per block of at most 32 consecutive rows (see
+// rows_per_warp).  Rows with
 // more than kLongRow entries are not summed here: the warp appends them to a
 // list (order immaterial) and leaves them to the second launch.
 //
@@ -154,56 +155,76 @@ __device__ __forceinline__ void spmv_block_rows(int r0, int nr, long long rs, lo
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kSpmvWarps * 32) spmv_rows32_kernel(
+__global__ void __launch_bounds__(kSpmvWarps * 32, sizeof(T) == 8 ? 6 : 0) spmv_rows_kernel(
     int m, const int64_t* __restrict__ rp, const int* __restrict__ ri,
     const T* __restrict__ rx, const T* __restrict__ x, T* __restrict__ y,
-    int* __restrict__ long_rows, int variant) {
+    int* __restrict__ long_rows, int rows_per_warp) {
   __shared__ T stage[kSpmvWarps][kStageEntries];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long nblk = ((long long)m + 31) / 32;
-  const long long stride = (long long)gridDim.x * kSpmvWarps;
-  for (long long b = (long long)blockIdx.x * kSpmvWarps + w; b < nblk; b += stride) {
-    const int r0 = (int)(b * 32);
-    const int nr = min(32, m - r0);
-    const long long rs = lane < nr ? (long long)__ldg(rp + r0 + lane) : 0LL;
-    const long long re = lane < nr ? (long long)__ldg(rp + r0 + lane + 1) : 0LL;
-    const bool is_long = lane < nr && re - rs > kLongRow;
-    if (is_long) {
-      // a count left over by a failed earlier call cannot push a write past
-      // the list (m + 2 entries): the slot is checked
-      const int slot = atomicAdd(long_rows, 1);
-      if (slot < m) long_rows[2 + slot] = r0 + lane;
-    }
-    const unsigned long_mask = __ballot_sync(kAll, is_long);
-    const unsigned rows_mask = nr == 32 ? kAll : ((1u << nr) - 1u);
-    unsigned skip = long_mask;                  // rows the row-group path leaves alone
-    if (variant != SPMV_ROW_GROUPS) {
-      // every short row, in runs that fit the buffer; long rows are left to
-      // the second launch
-      for (int start = 0; start < nr;) {
-        if ((long_mask >> start) & 1u) { ++start; continue; }
-        const int end = spmv_next_run(start, nr, rs, re, long_mask, lane);
-        const long long qa = __shfl_sync(kAll, rs, start), qb = __shfl_sync(kAll, re, end - 1);
-        spmv_rows_staged<T>(r0, start, end, rs, re, qa, (int)(qb - qa), lane, ri, rx, x, y,
-                            stage[w]);
-        start = end;
-      }
-      continue;
-    }
-    // mean length of the rows left -> lanes per row
-    const bool mine = lane < nr && !((skip >> lane) & 1u);
-    long long len = mine ? re - rs : 0;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) len += __shfl_xor_sync(kAll, len, off);
-    const int left = __popc(rows_mask & ~skip);
-    const long long avg = left > 0 ? (len + left - 1) / left : 0;
-    if (avg <= 1) spmv_block_rows<T, 1>(r0, nr, rs, re, skip, lane, ri, rx, x, y);
-    else if (avg <= 2) spmv_block_rows<T, 2>(r0, nr, rs, re, skip, lane, ri, rx, x, y);
-    else if (avg <= 4) spmv_block_rows<T, 4>(r0, nr, rs, re, skip, lane, ri, rx, x, y);
-    else if (avg <= 8) spmv_block_rows<T, 8>(r0, nr, rs, re, skip, lane, ri, rx, x, y);
-    else if (avg <= 16) spmv_block_rows<T, 16>(r0, nr, rs, re, skip, lane, ri, rx, x, y);
-    else spmv_block_rows<T, 32>(r0, nr, rs, re, skip, lane, ri, rx, x, y);
+  // both launches of a call are programmatic dependents of the launch before
+  // them: their blocks take their places on the SMs while it drains, and wait
+  // here until it has completed.  (This pass does not release the long-row
+  // launch early: its waiting blocks slowed the last wave, 52 us against 50.7 on
+  // a 600,000-row plan.)
+  grid_dep_wait();
+  const long long b = (long long)blockIdx.x * kSpmvWarps + w;
+  if (b * rows_per_warp >= m) return;               // whole warps leave together
+  const int r0 = (int)(b * rows_per_warp);
+  const int nr = min(rows_per_warp, m - r0);
+  const long long rs = lane < nr ? (long long)__ldg(rp + r0 + lane) : 0LL;
+  const long long re = lane < nr ? (long long)__ldg(rp + r0 + lane + 1) : 0LL;
+  const bool is_long = lane < nr && re - rs > kLongRow;
+  if (is_long) {
+    // a count left over by a failed earlier call cannot push a write past
+    // the list (m + 2 entries): the slot is checked
+    const int slot = atomicAdd(long_rows, 1);
+    if (slot < m) long_rows[2 + slot] = r0 + lane;
   }
+  const unsigned long_mask = __ballot_sync(kAll, is_long);
+  // every short row, in runs that fit the buffer; long rows are left to the
+  // second launch
+  for (int start = 0; start < nr;) {
+    if ((long_mask >> start) & 1u) { ++start; continue; }
+    const int end = spmv_next_run(start, nr, rs, re, long_mask, lane);
+    const long long qa = __shfl_sync(kAll, rs, start), qb = __shfl_sync(kAll, re, end - 1);
+    spmv_rows_staged<T>(r0, start, end, rs, re, qa, (int)(qb - qa), lane, ri, rx, x, y, stage[w]);
+    start = end;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSpmvWarps * 32) spmv_groups_kernel(
+    int m, const int64_t* __restrict__ rp, const int* __restrict__ ri,
+    const T* __restrict__ rx, const T* __restrict__ x, T* __restrict__ y,
+    int* __restrict__ long_rows) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  grid_dep_wait();
+  const long long b = (long long)blockIdx.x * kSpmvWarps + w;
+  if (b * 32 >= m) return;                          // whole warps leave together
+  const int r0 = (int)(b * 32);
+  const int nr = min(32, m - r0);
+  const long long rs = lane < nr ? (long long)__ldg(rp + r0 + lane) : 0LL;
+  const long long re = lane < nr ? (long long)__ldg(rp + r0 + lane + 1) : 0LL;
+  const bool is_long = lane < nr && re - rs > kLongRow;
+  if (is_long) {
+    const int slot = atomicAdd(long_rows, 1);
+    if (slot < m) long_rows[2 + slot] = r0 + lane;
+  }
+  const unsigned long_mask = __ballot_sync(kAll, is_long);
+  const unsigned rows_mask = nr == 32 ? kAll : ((1u << nr) - 1u);
+  // mean length of the short rows -> lanes per row
+  const bool mine = lane < nr && !is_long;
+  long long len = mine ? re - rs : 0;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) len += __shfl_xor_sync(kAll, len, off);
+  const int left = __popc(rows_mask & ~long_mask);
+  const long long avg = left > 0 ? (len + left - 1) / left : 0;
+  if (avg <= 1) spmv_block_rows<T, 1>(r0, nr, rs, re, long_mask, lane, ri, rx, x, y);
+  else if (avg <= 2) spmv_block_rows<T, 2>(r0, nr, rs, re, long_mask, lane, ri, rx, x, y);
+  else if (avg <= 4) spmv_block_rows<T, 4>(r0, nr, rs, re, long_mask, lane, ri, rx, x, y);
+  else if (avg <= 8) spmv_block_rows<T, 8>(r0, nr, rs, re, long_mask, lane, ri, rx, x, y);
+  else if (avg <= 16) spmv_block_rows<T, 16>(r0, nr, rs, re, long_mask, lane, ri, rx, x, y);
+  else spmv_block_rows<T, 32>(r0, nr, rs, re, long_mask, lane, ri, rx, x, y);
 }
 
 // Banded variant: one block per 256 consecutive rows (a warp per 32), no
@@ -222,6 +243,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_band_kernel(
   __shared__ T band[kBandCap];
   __shared__ int wlo[kSpmvWarps], whi[kSpmvWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  grid_dep_wait();
   const long long nblk = ((long long)m + 31) / 32;
   const long long b = (long long)blockIdx.x * kSpmvWarps + w;
   const bool have = b < nblk;                       // warp-uniform
@@ -278,6 +300,8 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_long_rows_kernel(
   __shared__ T part[kSpmvWarps];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  grid_dep_release();
+  grid_dep_wait();                  // the row-block pass has filled the list
   const int count = min(long_rows[0], m);
   for (int k = blockIdx.x; k < count; k += gridDim.x) {
     const int r = long_rows[2 + k];
@@ -352,6 +376,27 @@ int long_row_list(cudaStream_t st, size_t entries, int** out) {
   return PDLP_OK;
 }
 
+// Rows per warp of the streamed pass, 4 to 32: as many as leave
+// kSpmvTargetWarps warps (56 of an SM's 64).  A warp walks its rows' runs of
+// 256 entries one after another, so few long rows want few rows a warp, and
+// many rows want many, to fill the runs.  Float64 on B200, us per product with
+// 4 / 8 / 16 / 32 rows a warp: 50,000 rows of 39 entries 17 / 19 / 28 / 44; 100,000
+// of 15: 17.4 / 13.9 / 14.6 / 16.4; 200,000 of 15: 35 / 26.4 / 25.2 / 26.0; 300,000 of
+// 6: 33 / 20.8 / 16.1 / 15.1; 600,000 of 5: 65 / 38 / 27 / 22.1; 3,000,000 of 3: 311 /
+// 166 / 98 / 69.  64 rows a warp (two per lane) gained on uniform rows of 3
+// entries (58) and lost on power-law ones (float32 101 against 97) and on
+// 200,000 rows of 15 (40).  Each row's sum is the same whichever warp takes
+// it.  Six blocks per SM pay in float64 (40 registers: 74.4 and 99.5 us on the
+// power law's two products, 82.2 and 101.1 without the bound) and lose in
+// float32 (71.5 and 93.8 against 65.4 and 89.8).
+constexpr int kSpmvTargetWarps = 148 * 56;
+constexpr int kLongBlocks = 592;
+int rows_per_warp(int m) {
+  int r = 32;
+  while (r > 4 && (long long)m < (long long)r * kSpmvTargetWarps) r >>= 1;
+  return r;
+}
+
 template <typename T>
 int launch_spmv(int m, const int64_t* rp, const int* ri, const T* rx, const T* x, T* y,
                 cudaStream_t st, int variant = SPMV_AUTO) {
@@ -362,16 +407,26 @@ int launch_spmv(int m, const int64_t* rp, const int* ri, const T* rx, const T* x
   int* long_rows = nullptr;
   const int rc = long_row_list(st, (size_t)m + 2, &long_rows);
   if (rc != PDLP_OK) return rc;
-  const long long nblk = ((long long)m + 31) / 32;
-  const int g = (int)std::min((nblk + kSpmvWarps - 1) / kSpmvWarps, 1LL << 30);
-  if (variant == SPMV_BANDED) {
-    const long long gb = (nblk + kSpmvWarps - 1) / kSpmvWarps;
-    if (gb > (1LL << 31) - 1) return fail(PDLP_ERR_ARG, "m too large for the banded variant");
-    spmv_band_kernel<T><<<(int)gb, kSpmvWarps * 32, 0, st>>>(m, rp, ri, rx, x, y, long_rows);
-  } else {
-    spmv_rows32_kernel<T><<<g, kSpmvWarps * 32, 0, st>>>(m, rp, ri, rx, x, y, long_rows, variant);
-  }
-  spmv_long_rows_kernel<T><<<592, kSpmvWarps * 32, 0, st>>>(rp, ri, rx, x, y, m, long_rows);
+  const int rows = variant == SPMV_ROW_GROUPS || variant == SPMV_BANDED ? 32 : rows_per_warp(m);
+  const long long nblk = ((long long)m + rows - 1) / rows;
+  const long long g = (nblk + kSpmvWarps - 1) / kSpmvWarps;    // at most 2^31 / 32
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)g);
+  cfg.blockDim = dim3(kSpmvWarps * 32);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (variant == SPMV_BANDED)
+    PDLP_CUDA(cudaLaunchKernelEx(&cfg, spmv_band_kernel<T>, m, rp, ri, rx, x, y, long_rows));
+  else if (variant == SPMV_ROW_GROUPS)
+    PDLP_CUDA(cudaLaunchKernelEx(&cfg, spmv_groups_kernel<T>, m, rp, ri, rx, x, y, long_rows));
+  else
+    PDLP_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<T>, m, rp, ri, rx, x, y, long_rows, rows));
+  cfg.gridDim = dim3((unsigned)std::min(m, kLongBlocks));
+  PDLP_CUDA(cudaLaunchKernelEx(&cfg, spmv_long_rows_kernel<T>, rp, ri, rx, x, y, m, long_rows));
   count_launches(2);
   PDLP_CUDA(cudaGetLastError());
   return PDLP_OK;

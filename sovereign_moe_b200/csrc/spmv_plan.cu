@@ -187,19 +187,6 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-// Programmatic dependent launch.  grid_dep_wait returns once the kernel
-// before this one in the stream has completed and its writes are visible (at
-// once when there is none); grid_dep_release lets the next kernel in the
-// stream, if it was launched as a programmatic dependent, start its CTAs as
-// this kernel's CTAs leave the SMs.
-__device__ __forceinline__ void grid_dep_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-__device__ __forceinline__ void grid_dep_release() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Waits for the phase of `bar` with parity `parity`; false (and the status
 // word set) once kPlanWaitNs of wall time have passed.
 __device__ bool plan_wait(unsigned long long* bar, unsigned parity, int* status) {
