@@ -22,6 +22,21 @@ constexpr int kVecs = 7;               // vectors staged for a hot-mode epilogue
 constexpr double kRuizTol = 1e-2;      // scaling.py:149
 constexpr unsigned kFull = 0xffffffffu;
 
+// A warp's own copy of the scheduling fields of its team's LP, for teams of
+// one LP (persistent launches).  A normal iteration (an R_ITER pass, and a
+// C_ITER pass that ends in a normal primal step) reduces nothing, and the state
+// it leads to follows from these fields alone.  So every warp advances its
+// copy by itself: no counters, no finisher, no state writes and no reload.
+// `pend` counts the iterations the copy is ahead of the State in memory; the
+// next finisher, or the team's leader at the end of the launch, writes them
+// down first.  After every other pass the warps reload the copy.
+struct TeamCopy {
+  double eta, omega;
+  long long k;
+  int rmode, cmode, cprimal, xcommit, ycommit;
+  int pend;
+};
+
 // Per-warp shared memory.  The s* arrays receive bulk asynchronous copies
 // (whole 16-byte chunks) of a tile's row pointers, indices, values and
 // epilogue vectors; each has room for the alignment offset of the copied
@@ -35,10 +50,12 @@ struct __align__(16) WarpSmem {
   double vec[kVecs][kWTileRows + 4];
   double s0[kWTileRows];               // row sums, first right-hand side
   double s1[kWTileRows];               // row sums, second right-hand side
+  TeamCopy team;
   int inst_id;
   int pad[3];
   Inst inst;                           // cached descriptor of inst_id
 };
+static_assert(sizeof(TeamCopy) % 16 == 0, "WarpSmem layout");
 
 // ---- bulk asynchronous staging (cp.async.bulk + mbarrier) --------------------
 //
@@ -166,16 +183,45 @@ __device__ __forceinline__ void warp_reduce(double* v, Ops ops) {
 // storage order, then a xor butterfly; L == 1 is the storage-order sum).
 // Heavy tile (one row longer than a normal tile holds): the 32 lanes stride
 // over the row, then a xor butterfly.  Either way the order depends only on
-// the row and L.  term(p, rhs) returns value[p] * x_rhs[index[p]].
+// the row and L.  term(p, rhs) returns the factors value[p], x_rhs[index[p]].
+struct Factors {
+  double a, x;
+};
+constexpr int kHeavyLoads = 8;
+
 template <int NR, class F>
 __device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const int* tptr, int L,
                                           F term, WarpSmem& W, int lane) {
   if (t.heavy) {
     const int p0 = ld_ro(ptr + t.begin), p1 = ld_ro(ptr + t.begin + 1);
     double a0 = 0.0, a1 = 0.0;
-    for (int p = p0 + lane; p < p1; p += 32) {
-      a0 += term(p, 0);
-      if (NR == 2) a1 += term(p, 1);
+    // kHeavyLoads factors' loads of each lane in flight, added in order: a row of a
+    // thousand entries is a chain of 4 round trips instead of 32, which set
+    // the A pass of plans with coupling rows
+    constexpr int kU = kHeavyLoads / NR;
+    int p = p0 + lane;
+#pragma unroll 1
+    for (; p + 32 * (kU - 1) < p1; p += 32 * kU) {
+      Factors f[kU], g[NR == 2 ? kU : 1];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        f[u] = term(p + 32 * u, 0);
+        if (NR == 2) g[u] = term(p + 32 * u, 1);
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        a0 = fma(f[u].a, f[u].x, a0);
+        if (NR == 2) a1 = fma(g[u].a, g[u].x, a1);
+      }
+    }
+#pragma unroll 1
+    for (; p < p1; p += 32) {
+      const Factors f = term(p, 0);
+      a0 = fma(f.a, f.x, a0);
+      if (NR == 2) {
+        const Factors g = term(p, 1);
+        a1 = fma(g.a, g.x, a1);
+      }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -197,7 +243,11 @@ __device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const i
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int q = q0 + u * 32 + lane;
-        v[u] = q < cnt ? term(p0 + q, rhs) : 0.0;
+        v[u] = 0.0;
+        if (q < cnt) {
+          const Factors f = term(p0 + q, rhs);
+          v[u] = f.a * f.x;
+        }
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {

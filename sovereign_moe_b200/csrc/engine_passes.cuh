@@ -676,8 +676,8 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       auto term = [&](int p, int rhs) {
         const int j = ld_ro(ri + p);
         const double a = ld_mut(rx + p);
-        if (rhs == 0) return a * (scale != 0.0 ? ld_mut(v + j) / scale : 0.0);
-        return a * ld_mut(I.x + j);
+        if (rhs == 0) return Factors{a, scale != 0.0 ? ld_mut(v + j) / scale : 0.0};
+        return Factors{a, ld_mut(I.x + j)};
       };
       if (round == 1) warp_spmv<2>(t, rp, tptr, L, term, W, lane);
       else warp_spmv<1>(t, rp, tptr, L, term, W, lane);
@@ -698,7 +698,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* rx = I.rx;
       const double* dxv = I.dx;
       warp_spmv<1>(t, rp, tptr, L, [&](int p, int) {
-        return ld_mut(rx + p) * ld_mut(dxv + ld_ro(ri + p));
+        return Factors{ld_mut(rx + p), ld_mut(dxv + ld_ro(ri + p))};
       }, W, lane);
       for (int r = t.begin + lane; r < rend; r += 32) {
         do_commit(r);
@@ -720,7 +720,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* rx = I.rx;
       const double* dxv = I.dx;
       warp_spmv<1>(t, rp, tptr, L, [&](int p, int) {
-        return ld_mut(rx + p) * ld_mut(dxv + ld_ro(ri + p));
+        return Factors{ld_mut(rx + p), ld_mut(dxv + ld_ro(ri + p))};
       }, W, lane);
       for (int r = t.begin + lane; r < rend; r += 32) {
         do_commit(r);
@@ -763,7 +763,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* xc = I.x;
       warp_spmv<2>(t, rp, tptr, L, [&](int p, int rhs) {
         const int j = ld_ro(ri + p);
-        return ld_mut(rx + p) * ld_mut((rhs == 0 ? xb : xc) + j);
+        return Factors{ld_mut(rx + p), ld_mut((rhs == 0 ? xb : xc) + j)};
       }, W, lane);
       ops.maxmask = 7u;
       for (int r = t.begin + lane; r < rend; r += 32) {
@@ -1188,7 +1188,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* cx = I.cx;
       const double* av = I.ybar;
       warp_spmv<1>(t, cp, tptr, L, [&](int p, int) {
-        return ld_mut(cx + p) * ld_mut(av + ld_ro(ci + p));
+        return Factors{ld_mut(cx + p), ld_mut(av + ld_ro(ci + p))};
       }, W, lane);
       for (int j = t.begin + lane; j < rend; j += 32) {
         const double v = W.s0[j - t.begin];
@@ -1204,7 +1204,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const int kind = cprimal;
       const double* dyv = I.dy;
       warp_spmv<1>(t, cp, tptr, L, [&](int p, int) {
-        return ld_mut(cx + p) * ld_mut(dyv + ld_ro(ci + p));
+        return Factors{ld_mut(cx + p), ld_mut(dyv + ld_ro(ci + p))};
       }, W, lane);
       for (int j = t.begin + lane; j < rend; j += 32) {
         const double xv = xc ? ld_mut(I.xnew + j) : ld_mut(I.x + j);
@@ -1250,7 +1250,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* yc = I.y;
       warp_spmv<2>(t, cp, tptr, L, [&](int p, int rhs) {
         const int i = ld_ro(ci + p);
-        return ld_mut(cx + p) * ld_mut((rhs == 0 ? yb : yc) + i);
+        return Factors{ld_mut(cx + p), ld_mut((rhs == 0 ? yb : yc) + i)};
       }, W, lane);
       const double s = ld_mut(&S->s_obj);
       ops.maxmask = (1u << 0) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 6);
@@ -1294,7 +1294,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* ysrc = avg ? I.ybar : I.y;
       const double* cx = I.cx;
       warp_spmv<1>(t, cp, tptr, L, [&](int p, int) {
-        return ld_mut(cx + p) * ld_mut(ysrc + ld_ro(ci + p));
+        return Factors{ld_mut(cx + p), ld_mut(ysrc + ld_ro(ci + p))};
       }, W, lane);
       const double s = ld_mut(&S->s_obj);
       const double dsign = I.sense == 1 ? 1.0 : -1.0;
