@@ -31,8 +31,14 @@ namespace pdlp {
 // barrier's acquire nor a __threadfence orders generic writes before async-
 // proxy reads, so the caller follows every barrier with a global proxy fence
 // in each thread that issues copies (fence_proxy_async_global).
-__device__ bool grid_barrier(Control* ctl, unsigned* counter, unsigned target,
-                             long long timeout_ns, int* flag, bool alone, bool withhold) {
+// A set kStopBit in the counter (added by a team's leader with its arrival)
+// tells every block of the team, at the same barrier, to leave after the step.
+constexpr unsigned kStopBit = 0x40000000u;
+
+// Returns 0 to leave the kernel, else 1, or 3 when the stop bit is set.
+__device__ int grid_barrier(Control* ctl, unsigned* counter, unsigned target,
+                            long long timeout_ns, bool alone, bool withhold, unsigned add) {
+  volatile int* const flags = block_flags();
   __syncthreads();
   if (alone) {
     // A team of one block: no other block waits for it.  The __syncthreads
@@ -41,21 +47,24 @@ __device__ bool grid_barrier(Control* ctl, unsigned* counter, unsigned target,
     // ld.global.cg) as the release of a multi-block barrier does.
     if (threadIdx.x == 0) {
       __threadfence();
-      *flag = *(volatile int*)&ctl->error == 0;
+      flags[0] = flags[1] ? 0 : (add & kStopBit) ? 3 : 1;
     }
     __syncthreads();
-    return *flag != 0;
+    return flags[0];
   }
   // test hook: this block leaves without arriving; the rest of the team waits
   // until the bounded wait below runs out
-  if (withhold) return false;
+  if (withhold) return 0;
   if (threadIdx.x == 0) {
     volatile int* err = &ctl->error;
-    int ok = 1;
-    if (atom_add_acq_rel(counter, 1u) + 1u < target) {
+    // read before the arrival, so that its round trip is the arrival's: an
+    // error set later is seen at the next barrier, or in the wait
+    int ok = *err == 0 && flags[1] == 0;
+    unsigned v = atom_add_acq_rel(counter, add) + add;
+    if ((v & (kStopBit - 1u)) < target) {
       const long long t0 = global_ns();
       unsigned spins = 0;
-      while (ld_acquire(counter) < target) {
+      while (((v = ld_acquire(counter)) & (kStopBit - 1u)) < target) {
         if ((++spins & 255u) == 0u) {
           if (*err != 0) { ok = 0; break; }
           if (global_ns() - t0 > timeout_ns) {
@@ -66,10 +75,10 @@ __device__ bool grid_barrier(Control* ctl, unsigned* counter, unsigned target,
         }
       }
     }
-    *flag = ok && (*err == 0);
+    flags[0] = ok ? ((v & kStopBit) ? 3 : 1) : 0;
   }
   __syncthreads();
-  return *flag != 0;
+  return flags[0];
 }
 
 // One launch runs up to max_steps engine steps; every warp owns a fixed range
@@ -78,16 +87,18 @@ __device__ bool grid_barrier(Control* ctl, unsigned* counter, unsigned target,
 // its own instances, and its barriers count only its blocks.  A team stops
 // when its instances are done, after max_steps, or when another team has
 // stopped (the host then re-plans the teams for what is left).  The team's
-// first block decides each next step between the step's two barriers, so
-// that every block of the team sees the same decision.
-extern __shared__ __align__(16) unsigned char g_smem[];
-constexpr size_t kSmemBytes = sizeof(WarpSmem) * kWarps + 16;
-
+// first block decides each next step at the step's second barrier, so that
+// every block of the team sees the same decision.
+//
+// A team of one LP (team_inst) keeps the LP's scheduling fields in its warps
+// (TeamCopy).  Its normal iterations then cost two barriers and nothing else:
+// no counters, no finisher, no state read.  Alone, in us per iteration with
+// checks and set-up: a 3 x 5 LP 16.2 -> 13.0, 230 x 2,025 20.4 -> 17.9.
 __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
   WarpSmem* ws = reinterpret_cast<WarpSmem*>(g_smem);
-  int& flag = *reinterpret_cast<int*>(g_smem + sizeof(WarpSmem) * kWarps);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSmem& W = ws[warp];
+  if (threadIdx.x == 0) block_flags()[1] = 0;
   if (lane == 0) {
     W.inst_id = -1;
     mbar_init(&W.bar[0]);
@@ -107,7 +118,14 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
   unsigned* const bar = &A.ctl->team_bar[team];
   const unsigned nb = (unsigned)A.team_blocks[team];
   const bool withhold = (int)blockIdx.x == A.withhold_block;
-  const long long budget = *(volatile int*)&A.ctl->team_budget[team];
+  const int budget = *(volatile int*)&A.ctl->team_budget[team];
+  const int inst = A.team_inst[team];              // the team's only LP, or -1
+  State* const S = A.st + max(inst, 0);
+  TeamCopy& C = W.team;
+  if (inst >= 0) {
+    warp_inst(A, inst, W, lane);
+    team_load(C, S, lane);
+  }
   unsigned target = 0;
 #ifdef PDLP_TRACE
   // phase timestamps of the first and the last block for the first steps
@@ -118,49 +136,78 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
 #else
 #define PDLP_STAMP(step, k)
 #endif
-  long long step = 0;
+  int step = 0;
   for (; step < budget; ++step) {
-    if (threadIdx.x == 0)
-      flag = *(volatile int*)&A.ctl->team_active[team] > 0 &&
-             *(volatile int*)&A.ctl->team_go[team] != 0;
-    __syncthreads();
-    if (!flag) break;
-    __syncthreads();
+    if (inst >= 0) {
+      if (C.rmode == R_NONE && C.cmode == C_NONE) break;     // the LP is done
+    } else {
+      if (threadIdx.x == 0) block_flags()[2] = *(volatile int*)&A.ctl->team_active[team] > 0;
+      __syncthreads();
+      if (!block_flags()[2]) break;
+      __syncthreads();
+    }
     PDLP_STAMP(step, 0);
-    {
+    // the leader's decision for the next step travels with its arrival at the
+    // step's second barrier; the flag's round trip overlaps the passes
+    const int stop = leader && threadIdx.x == 0 ? *(volatile int*)&A.ctl->stop : 0;
+    if (inst < 0 || C.rmode != R_NONE) {           // a team of one LP skips an empty A pass
       Tile next = rfirst;
       PassCache pc;
+      if (inst >= 0) pc.copy(inst, C.rmode, 0, C.ycommit, C.eta, C.omega);
       for (int t = r0; t < r1; ++t) {
         const Tile cur = next;
         if (t + 1 < r1) next = A.rtiles[t + 1];      // prefetch the next descriptor
         ph.flush = t + 1 >= r1 || next.group != cur.group;
-        process_rtile(A, cur, t, W, lane, pc, ph);
+        process_rtile(A, cur, t, W, lane, pc, ph, inst >= 0 ? &C : nullptr);
+      }
+      PDLP_STAMP(step, 1);
+      target += nb;
+      if (!grid_barrier(A.ctl, bar, target, A.barrier_timeout_ns, nb == 1u, withhold, 1u)) return;
+      if (lane == 0) fence_proxy_async_global();
+      if (inst >= 0) {
+        if (C.rmode != R_ITER) team_load(C, S, lane);
+        else {
+          __syncwarp();
+          if (lane == 0) C.ycommit = 0;              // this pass has retired it
+          __syncwarp();
+        }
       }
     }
-    PDLP_STAMP(step, 1);
-    target += nb;
-    if (!grid_barrier(A.ctl, bar, target, A.barrier_timeout_ns, &flag, nb == 1u, withhold)) return;
-    if (lane == 0) fence_proxy_async_global();
     PDLP_STAMP(step, 2);
-    // the leader's decision for the next step, published by its arrival at
-    // the next barrier
-    if (leader && threadIdx.x == 0)
-      A.ctl->team_go[team] = *(volatile int*)&A.ctl->stop == 0;
+    const bool quiet = inst >= 0 && C.cmode == C_ITER && C.cprimal == P_NORMAL;
     {
       Tile next = cfirst;
       PassCache pc;
+      if (inst >= 0) pc.copy(inst, C.cmode, C.cprimal, C.xcommit, C.eta, C.omega);
       for (int t = c0; t < c1; ++t) {
         const Tile cur = next;
         if (t + 1 < c1) next = A.ctiles[t + 1];
         ph.flush = t + 1 >= c1 || next.group != cur.group;
-        process_ctile(A, cur, t, W, lane, pc, ph);
+        process_ctile(A, cur, t, W, lane, pc, ph, inst >= 0 ? &C : nullptr, quiet);
       }
     }
     PDLP_STAMP(step, 3);
     target += nb;
-    if (!grid_barrier(A.ctl, bar, target, A.barrier_timeout_ns, &flag, nb == 1u, withhold)) return;
+    const int go = grid_barrier(A.ctl, bar, target, A.barrier_timeout_ns, nb == 1u, withhold,
+                                stop ? 1u + kStopBit : 1u);
+    if (!go) return;
     if (lane == 0) fence_proxy_async_global();
+    if (quiet) {
+      // the next state, as c_finish computes it for a normal step
+      __syncwarp();
+      if (lane == 0) {
+        C.xcommit = 0;
+        C.k += 1;
+        C.pend += 1;
+        C.cprimal = plan_primal(W.inst, C.k + 1);
+        C.rmode = R_ITER;
+      }
+      __syncwarp();
+    } else if (inst >= 0 && C.cmode != C_NONE) {
+      team_load(C, S, lane);
+    }
     PDLP_STAMP(step, 4);
+    if (go & 2) { ++step; break; }
   }
   // This team is done for the launch; its leader reports the steps it ran.
   // After the launch's step cap the launch ends (the other teams leave at
@@ -169,7 +216,8 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
   // ends the launch once an eighth of the blocks are idle, so that the host
   // can give them to what is left without re-planning at every finish.
   if (leader && threadIdx.x == 0) {
-    A.ctl->team_steps[team] = (int)step;
+    if (inst >= 0) team_flush(C, S);
+    A.ctl->team_steps[team] = step;
     if (step == A.max_steps) {
       atomicExch(&A.ctl->stop, 1);
     } else if (step < budget && *(volatile int*)&A.ctl->team_active[team] <= 0) {
@@ -197,9 +245,9 @@ __global__ void __launch_bounds__(kBlock, 3) engine_pass(EngineArgs A, int side)
   PassCache pc;
   BulkPhase ph;
   if (side == 0) {
-    for (int t = gw; t < A.n_rtiles; t += nw) process_rtile(A, A.rtiles[t], t, W, lane, pc, ph);
+    for (int t = gw; t < A.n_rtiles; t += nw) process_rtile(A, A.rtiles[t], t, W, lane, pc, ph, nullptr);
   } else {
-    for (int t = gw; t < A.n_ctiles; t += nw) process_ctile(A, A.ctiles[t], t, W, lane, pc, ph);
+    for (int t = gw; t < A.n_ctiles; t += nw) process_ctile(A, A.ctiles[t], t, W, lane, pc, ph, nullptr, false);
   }
 }
 
@@ -736,11 +784,19 @@ static double expected_left(const pdlp_batch* b, int s) {
   return -1.0;
 }
 
+// The most blocks an instance can use: a warp's tile gathers 512 scattered
+// doubles, and the warps of an SM share its load units, so two tiles a block
+// on twice the SMs finish a pass sooner than one per warp (10,000 x 40,000 in
+// float32 alone, us per iteration: four tiles a block 28.2, two 22.3, one 23.6 --
+// more blocks also mean more arrivals at the barriers; 35 LPs of up to 1,500
+// rows: 111, 98 and 96 ms).
+constexpr int kTilesPerBlock = 2;
+
 // The block teams of a persistent launch.  With many running instances one
 // team of blocks steps them all.  With fewer (at most kTeamsFrom), each
 // instance gets its own team, so that no instance waits at a barrier for
 // another's tiles.  Teams get blocks in proportion to each instance's weight,
-// but never more than one tile per warp can use: the blocks an instance
+// but never more than leave kTilesPerBlock tiles a block: the blocks an instance
 // cannot use go to the others (water-filling), and the blocks left by
 // rounding go to the largest remainders.  The weight is the instance's work
 // per iteration, times the square root of its expected remaining iterations
@@ -778,7 +834,7 @@ static std::vector<int> plan_teams(const pdlp_batch* b, const std::vector<int>& 
     if (hinted) per *= std::sqrt(left[k]);
     w[k] = per;
     const int tiles = std::max(sl.inst.rt_end - sl.inst.rt_begin, sl.inst.ct_end - sl.inst.ct_begin);
-    want[k] = std::max(1, (tiles + kWarps - 1) / kWarps);    // one tile per warp
+    want[k] = std::max(1, (tiles + kTilesPerBlock - 1) / kTilesPerBlock);
   }
   tblocks.assign(T, 0);
   std::vector<char> full(T, 0);
@@ -868,7 +924,7 @@ static int rebuild(pdlp_batch* b) {
   const int max_blocks = std::max(1, b->sms * b->coop_blocks_per_sm);
   const std::vector<int> tblocks = plan_teams(b, run, max_blocks);
   // per warp tile ranges, then the team arrays: block_team[G], team_blocks[T],
-  // team_first[T]
+  // team_first[T], team_inst[T]
   std::vector<int> rwr, cwr, teams;
   if (tblocks.empty()) {
     std::vector<double> rw, cw;                 // one team splits every running tile
@@ -879,7 +935,7 @@ static int rebuild(pdlp_batch* b) {
       rw.insert(rw.end(), sl.rtw.begin(), sl.rtw.end());
       cw.insert(cw.end(), sl.ctw.begin(), sl.ctw.end());
     }
-    const int want = (std::max(b->n_rtiles, b->n_ctiles) + kWarps - 1) / kWarps;
+    const int want = (std::max(b->n_rtiles, b->n_ctiles) + kTilesPerBlock - 1) / kTilesPerBlock;
     int G = std::max(1, std::min(max_blocks, want));
     if (b->force_blocks > 0) G = std::min(G, b->force_blocks);
     b->grid = G;
@@ -890,6 +946,7 @@ static int rebuild(pdlp_batch* b) {
     teams.assign(G, 0);
     teams.push_back(G);
     teams.push_back(0);
+    teams.push_back(run.size() == 1 ? run[0] : -1);
     b->team_running.assign(1, (int)run.size());
     for (int s : run) b->slots[s].inst.team = 0;
   } else {
@@ -922,6 +979,7 @@ static int rebuild(pdlp_batch* b) {
     cwr.push_back(b->n_ctiles);
     for (int k = 0; k < T; ++k) teams.push_back(tblocks[k]);
     for (int k = 0; k < T; ++k) teams.push_back(first[k]);
+    for (int k = 0; k < T; ++k) teams.push_back(run[k]);
     b->team_running.assign(T, 1);
   }
   const size_t ngr = (size_t)b->n_groups;
@@ -1765,6 +1823,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     A.block_team = b->d_teams;
     A.team_blocks = b->d_teams + b->grid;
     A.team_first = b->d_teams + b->grid + b->n_teams;
+    A.team_inst = b->d_teams + b->grid + 2 * b->n_teams;
     A.group_tiles = b->d_group_tiles; A.n_rgroups = b->n_rgroups; A.n_groups = b->n_groups;
     A.partials = b->d_partials; A.gpartials = b->d_gpartials; A.gcounters = b->d_gcounters;
     const int64_t chunk = std::min(most, kChunk);
@@ -1774,7 +1833,6 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     b->h_ctl->error = 0; b->h_ctl->error_where = 0; b->h_ctl->stop = 0; b->h_ctl->idle = 0;
     for (int t = 0; t < kMaxTeams; ++t) {
       b->h_ctl->team_bar[t] = 0;
-      b->h_ctl->team_go[t] = 1;
       b->h_ctl->team_active[t] = t < (int)b->team_running.size() ? b->team_running[t] : 0;
       b->h_ctl->team_budget[t] = 0;
       b->h_ctl->team_steps[t] = 0;

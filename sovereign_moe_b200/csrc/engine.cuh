@@ -170,7 +170,6 @@ struct Control {
   unsigned int pad;
   unsigned int team_bar[kMaxTeams];   // each team's barrier arrival counter
   int team_active[kMaxTeams];         // each team's instances still running
-  int team_go[kMaxTeams];             // the team leader's decision for the next step
   int team_budget[kMaxTeams];         // steps each team may run in this launch (host)
   int team_steps[kMaxTeams];          // steps each team completed (its leader, at exit)
 };
@@ -185,6 +184,7 @@ struct EngineArgs {
   const int* block_team;    // persistent: team of each block
   const int* team_blocks;   // [n_teams] blocks per team
   const int* team_first;    // [n_teams] first block of each team (its leader)
+  const int* team_inst;     // [n_teams] the team's only instance, -1 for a team of several
   const int2* group_tiles;  // [n_groups]: tile range of each group (row groups first)
   int n_rgroups, n_groups;
   double* partials;         // [(n_rtiles + n_ctiles) * kNP] tile partials

@@ -52,6 +52,48 @@ __device__ __forceinline__ double merit(double omega, double p, double d, double
   return sqrt((omega * p) * (omega * p) + (d / omega) * (d / omega) + g * g);
 }
 
+// ---- teams of one LP: the warps' copies of its scheduling fields -------------
+
+__device__ __forceinline__ void team_load(TeamCopy& c, const State* S, int lane) {
+  __syncwarp();
+  if (lane == 0) {
+    const double eta = ld_mut(&S->eta), omega = ld_mut(&S->omega);
+    const long long k = ld_mut(&S->k);
+    const int rmode = ld_mut(&S->rmode), cmode = ld_mut(&S->cmode), cprimal = ld_mut(&S->cprimal);
+    const int xcommit = ld_mut(&S->xcommit), ycommit = ld_mut(&S->ycommit);
+    c.eta = eta;
+    c.omega = omega;
+    c.k = k;
+    c.rmode = rmode;
+    c.cmode = cmode;
+    c.cprimal = cprimal;
+    c.xcommit = xcommit;
+    c.ycommit = ycommit;
+    c.pend = 0;
+  }
+  __syncwarp();
+}
+
+// Writes down what the copy is ahead of the state: its normal iterations, one
+// addition to sum_eta each, as c_finish makes them, and the modes they lead
+// to.  By one thread, when every tile of those iterations has completed.
+__device__ void team_flush(const TeamCopy& c, State* S) {
+  if (c.pend > 0) {
+    const double eta = S->eta;
+    double sum = S->sum_eta;
+    for (int i = 0; i < c.pend; ++i) sum += eta;
+    S->sum_eta = sum;
+    S->k += c.pend;
+    S->epoch += c.pend;
+    S->iters_done += c.pend;
+    S->xcommit = 0;
+    S->cprimal = c.cprimal;
+    S->rmode = R_ITER;
+    S->cmode = C_ITER;
+  }
+  S->ycommit = c.ycommit;
+}
+
 // ---- finisher protocol ------------------------------------------------------
 //
 // Two-level, fixed-order reduction of an instance's tile partials: the warp
@@ -107,12 +149,20 @@ __device__ __forceinline__ bool warp_finish(const EngineArgs& A, const Tile& t, 
       for (int s = 0; s < kNP; ++s) v[s] = combine(v[s], ld_mut(tp + (size_t)tt * kNP + s), ops.op(s));
     }
     warp_reduce(v, ops);
-    if (lane == 0) {
+    if (lane == 0 && g_last - g_first > 1) {
 #pragma unroll
       for (int s = 0; s < kNP; ++s) A.gpartials[(size_t)g * kNP + s] = v[s];
     }
   }
   __syncwarp();
+  if (g_last - g_first == 1) {
+    // the instance's only group: its sums are the instance's (the second
+    // level would add them to zeros)
+    if (lane == 0) A.gcounters[g] = 0;
+#pragma unroll
+    for (int s = 0; s < kNP; ++s) res[s] = v[s];
+    return true;
+  }
   if (lane == 0) {
     A.gcounters[g] = 0;
     last = atom_add_acq_rel(A.counters + 2 * t.inst + side, 1u) == (unsigned)(g_last - g_first - 1);
@@ -160,6 +210,15 @@ struct PassCache {
   int inst = -1;
   int mode = 0, aux = 0, commit = 0;
   double eta = 0.0, omega = 0.0;
+  // from a warp's own copy (TeamCopy)
+  __device__ void copy(int id, int m, int a, int c, double e, double o) {
+    inst = id;
+    mode = m;
+    aux = a;
+    commit = c;
+    eta = e;
+    omega = o;
+  }
   __device__ void load_r(const State* S, int id) {
     inst = id;
     mode = ld_mut(&S->rmode);
@@ -248,6 +307,7 @@ __device__ void c_finish(const EngineArgs& A, const Inst& I, State* S, int cmode
 __device__ __forceinline__ bool index_ok(const EngineArgs& A, int i, int n, int where) {
   if ((unsigned)i < (unsigned)n) return true;
   if (atomicCAS(&A.ctl->error, 0, PDLP_ERR_BOUNDS) == 0) A.ctl->error_where = where;
+  block_fail();
   return false;
 }
 // The staged row pointers of a normal tile: start at the tile's first entry,
@@ -259,8 +319,10 @@ __device__ __forceinline__ bool tile_ptrs_ok(const EngineArgs& A, const Tile& t,
   for (int i = lane; i < rows; i += 32) ok &= tptr[i] <= tptr[i + 1];
   if (lane == 0) ok &= tptr[0] == t.p0 && tptr[rows] == t.p0 + t.cnt;
   ok = __all_sync(0xffffffffu, ok);
-  if (!ok && lane == 0 && atomicCAS(&A.ctl->error, 0, PDLP_ERR_BOUNDS) == 0)
-    A.ctl->error_where = t.begin;
+  if (!ok && lane == 0) {
+    if (atomicCAS(&A.ctl->error, 0, PDLP_ERR_BOUNDS) == 0) A.ctl->error_where = t.begin;
+    block_fail();
+  }
   return ok;
 }
 #else
@@ -322,6 +384,7 @@ __device__ bool bulk_wait(const EngineArgs& A, unsigned long long* bar, unsigned
       ok = mbar_try_wait(bar, parity);
       if (!ok && (spins & 63u) == 0u && global_ns() - t0 > A.barrier_timeout_ns) {
         atomicCAS(&A.ctl->error, 0, PDLP_ERR_BARRIER_TIMEOUT);
+        block_fail();
         break;
       }
     }
@@ -332,7 +395,8 @@ __device__ bool bulk_wait(const EngineArgs& A, unsigned long long* bar, unsigned
 
 __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst& I, State* S,
                           WarpSmem& W, int lane, int rmode, bool commit, double eta,
-                          double omega, int offp, int offi, int offv, BulkPhase& ph) {
+                          double omega, int offp, int offi, int offv, BulkPhase& ph,
+                          const TeamCopy* team) {
 #ifdef PDLP_TRACE
   // stage timestamps of the first warp of block 0 (slots after the step trace)
   // counter in trace[1279], records at trace[640 + 8 k], k < 63
@@ -425,7 +489,8 @@ __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst
 #endif
 #undef HOT_STAMP
   const bool need_red = rmode == R_TRIAL;
-  const bool need_fin = need_red || commit;
+  // a team of one LP retires a commit in its copies (TeamCopy)
+  const bool need_fin = need_red || (commit && team == nullptr);
   Ops ops;
   if (need_red) {
     warp_reduce(acc, ops);
@@ -438,7 +503,10 @@ __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst
   double res[kNP];
   if (warp_finish(A, t, 0, I.rg_begin, I.rg_end, I.rt_end - I.rt_begin, need_red, ops, res,
                   lane, ph)) {
-    if (lane == 0) r_finish(A, I, S, rmode, res);
+    if (lane == 0) {
+      if (team) team_flush(*team, S);
+      r_finish(A, I, S, rmode, res);
+    }
     __syncwarp();
   }
 }
@@ -446,7 +514,7 @@ __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst
 __device__ void hot_ctile(const EngineArgs& A, const Tile& t, int ti, const Inst& I, State* S,
                           WarpSmem& W, int lane, int cmode, int cprimal, bool xcommit,
                           double eta, double omega, int offp, int offi, int offv,
-                          BulkPhase& ph) {
+                          BulkPhase& ph, const TeamCopy* team, bool quiet) {
   const int rows = t.end - t.begin;
   const double tau = eta / omega;
   const bool iter = cmode == C_ITER;
@@ -505,6 +573,7 @@ __device__ void hot_ctile(const EngineArgs& A, const Tile& t, int ti, const Inst
       }
     }
   }
+  if (quiet) return;
   const bool need_red = cprimal == P_TRIAL;
   Ops ops;
   if (need_red) {
@@ -517,13 +586,18 @@ __device__ void hot_ctile(const EngineArgs& A, const Tile& t, int ti, const Inst
   double res[kNP];
   if (warp_finish(A, t, 1, I.cg_begin, I.cg_end, I.ct_end - I.ct_begin, need_red, ops, res,
                   lane, ph)) {
-    if (lane == 0) c_finish(A, I, S, cmode, res);
+    if (lane == 0) {
+      if (team) team_flush(*team, S);
+      c_finish(A, I, S, cmode, res);
+    }
     __syncwarp();
   }
 }
 
+// `team`: this warp's copy of the scheduling fields when its team steps one LP
+// (the pass cache then holds them), else null.
 __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSmem& W, int lane,
-                              PassCache& pc, BulkPhase& ph) {
+                              PassCache& pc, BulkPhase& ph, const TeamCopy* team) {
 #ifdef PDLP_TRACE
   if (A.trace && blockIdx.x == 0 && threadIdx.x == 0) {
     const long long k = A.trace[1279];
@@ -556,7 +630,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
     offv = I.f32 ? bulk_offset<4>(t.p0) : bulk_offset<8>(t.p0);
   }
   if ((rmode == R_ITER || rmode == R_TRIAL) && !t.heavy) {
-    hot_rtile(A, t, ti, I, S, W, lane, rmode, commit, eta, omega, offp, offi, offv, ph);
+    hot_rtile(A, t, ti, I, S, W, lane, rmode, commit, eta, omega, offp, offi, offv, ph, team);
     return;
   }
   if (!t.heavy && !bulk_wait(A, &W.bar[0], ph.m)) return;
@@ -808,7 +882,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
   // pending commit; the other modes reduce and/or advance the state machine.
   const bool need_red = rmode == R_RUIZ || rmode == R_APPLY || rmode == R_POWER ||
                         rmode == R_TRIAL || rmode == R_CHECK_A || rmode == R_CHECK_B;
-  const bool need_fin = !(rmode == R_ITER && !commit);
+  const bool need_fin = !(rmode == R_ITER && (!commit || team != nullptr));
   if (need_red) {
     warp_reduce(acc, ops);
     if (lane == 0) {
@@ -820,7 +894,10 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
   double res[kNP];
   if (warp_finish(A, t, 0, I.rg_begin, I.rg_end, I.rt_end - I.rt_begin, need_red, ops, res,
                   lane, ph)) {
-    if (lane == 0) r_finish(A, I, S, rmode, res);
+    if (lane == 0) {
+      if (team) team_flush(*team, S);
+      r_finish(A, I, S, rmode, res);
+    }
     __syncwarp();
   }
 }
@@ -1033,8 +1110,10 @@ __device__ void c_finish(const EngineArgs& A, const Inst& I, State* S, int cmode
   }
 }
 
+// `quiet`: a pass of a normal iteration in a team of one LP, with nothing to
+// finish (TeamCopy).
 __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSmem& W, int lane,
-                              PassCache& pc, BulkPhase& ph) {
+                              PassCache& pc, BulkPhase& ph, const TeamCopy* team, bool quiet) {
   State* S = A.st + t.inst;
   const Inst& I = warp_inst(A, t.inst, W, lane);
   if (pc.inst != t.inst) pc.load_c(S, t.inst);
@@ -1064,7 +1143,8 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
     offv = I.f32 ? bulk_offset<4>(t.p0) : bulk_offset<8>(t.p0);
   }
   if (hot) {
-    hot_ctile(A, t, ti, I, S, W, lane, cmode, cprimal, xcommit, eta, omega, offp, offi, offv, ph);
+    hot_ctile(A, t, ti, I, S, W, lane, cmode, cprimal, xcommit, eta, omega, offp, offi, offv, ph,
+              team, quiet);
     return;
   }
   if (!t.heavy && !bulk_wait(A, &W.bar[0], ph.m)) return;
@@ -1311,6 +1391,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
     default: break;
   }
 
+  if (quiet) return;
   const bool trial = (cmode == C_ITER || cmode == C_PRIMAL || cmode == C_RESTART) &&
                      cprimal == P_TRIAL;
   const bool need_red = trial || cmode == C_RUIZ || cmode == C_APPLY || cmode == C_SETUP0 ||
@@ -1327,7 +1408,10 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
   double res[kNP];
   if (warp_finish(A, t, 1, I.cg_begin, I.cg_end, I.ct_end - I.ct_begin, need_red, ops, res,
                   lane, ph)) {
-    if (lane == 0) c_finish(A, I, S, cmode, res);
+    if (lane == 0) {
+      if (team) team_flush(*team, S);
+      c_finish(A, I, S, cmode, res);
+    }
     __syncwarp();
   }
 }
