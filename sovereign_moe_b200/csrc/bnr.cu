@@ -7,11 +7,12 @@
 //
 // Layout: every per-node block is (rows, K) with the node index fastest, so a
 // sparse product reads A once for all K nodes (A X with X (n, K)).  One
-// iteration is five launches:
-//   primal step (+ sum dX dX)  ->  A dX  ->  dual step (+ sums dY AdX, dY dY)
-//   ->  A^T dY  ->  per-node accept / step size.
+// iteration is three launches, each a programmatic dependent of the one before:
+//   A^T dY and the primal step (+ sum dX dX)  ->  A dX and the dual step
+//   (+ sums dY AdX, dY dY)  ->  per-node accept / step size,
+// or, for wide batches, five, with the two products on their own.
 // A taken trial is not stored but redone by the next step, which reads the
-// same inputs anyway (see bnr_primal).
+// same inputs anyway (see bnr_cols).
 // The iterations of one call are captured once into a CUDA graph, keyed by
 // (K, iterations, step exponents), and replayed.
 //
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(256, 8) bnr_spmm(int rows, int k, const int64_
                                                 const double* __restrict__ X,
                                                 double* __restrict__ Y) {
   constexpr int kBatch = 2;
+  grid_dep_wait();
   const int groups = k / V;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (long long)rows * groups) return;
@@ -118,15 +120,294 @@ __global__ void __launch_bounds__(256, 8) bnr_spmm(int rows, int k, const int64_
   out.store(Y + r * k + col);
 }
 
+// ---- one iteration: a product fused with the step that uses it -----------------
+//
+// A block takes 64 consecutive rows and a tile of at most 16 nodes: 2^txs
+// threads along the nodes, V nodes each (two when K is even: 16-byte gathers
+// and vectors), the others along the rows.  Before it waits for the launch
+// before it (programmatic dependent launch) it stages the rows' pointers,
+// indices and values, which no launch changes, in shared memory; then the
+// gathers of the product and the vectors of the step are in flight together,
+// and the product goes to memory only where a later step needs it.
+//
+// Small batches are bound by the chain of launches and round trips: five
+// launches per iteration (primal, A dX, dual, A^T dY, accept) took 23 to 31 us
+// whatever the size; three take 10 to 20.  Per 60 iterations, split against
+// fused on B200: 2,000 x 3,000, 8 nodes 1.50 / 0.68 ms, 64 nodes 1.42 / 0.97;
+// 20,000 x 30,000, 8 nodes 1.86 / 1.26, 16 nodes 1.91 / 1.67.  Wide batches are
+// bound by the gathers, which L2 serves (245 MB per product at 128 nodes), and
+// want the most warps, which the split kernels have: 128 nodes 8.14 / 8.4 ms at
+// best.  See fused_shape for the line between them.
+//
 // The per-node sums over rows run in a fixed order: blocks of kRowsPerBlock
-// rows; in a block, phase y (threadIdx.y, 8 phases) adds rows r0 + y + 8 j
-// for j ascending from 0.0; the phases are added in order; then
-// warp_blocks_sum adds the blocks.  The element-wise kernels below walk their rows in that
-// layout, block (32, 8) with threadIdx.x the node within a 32-node tile, and
-// sum as they go.  Output pair of row block b and node j at
-// part[2 (j pstride + b)], pstride = mblocks + nblocks + 1, so one node's
-// partials are contiguous for the warp that adds them: m-side blocks
+// rows; in a block, phase p (8 phases) adds rows r0 + p + 8 j for j ascending
+// from 0.0; the phases are added in order; then bnr_accept adds the blocks.
+// The rows' terms go through shared memory.  Output pair of row block b and
+// node j at part[2 (j pstride + b)], pstride = mblocks + nblocks + 1, so one
+// node's partials are contiguous for the warp that adds them: m-side blocks
 // [0, mblocks), n-side blocks [mblocks, mblocks + nblocks).
+constexpr int kStageCap = 1024;      // entries of a block's rows that are staged
+constexpr int kBnrThreads = 256;
+constexpr int kTileNodes = 16;       // nodes of a block's tile, at most
+
+struct BnrStage {
+  double term[2][kRowsPerBlock * kTileNodes];   // the sums' terms: [row * tile + node]
+  int off[kRowsPerBlock + 1];        // from the block's first entry (nnz fits an int)
+  double val[kStageCap];
+  int idx[kStageCap];
+};
+
+template <int V>
+struct BnrTile {
+  int x, y, ty, tile, node, nr;      // thread's place, node tile width, first node, rows
+  bool live;
+};
+
+template <int V>
+__device__ __forceinline__ BnrTile<V> bnr_tile(int rows, int k, int txs) {
+  BnrTile<V> t;
+  t.x = threadIdx.x & ((1 << txs) - 1);
+  t.y = threadIdx.x >> txs;
+  t.ty = kBnrThreads >> txs;
+  t.tile = V << txs;
+  t.node = (blockIdx.y << txs) * V + t.x * V;
+  t.nr = min(kRowsPerBlock, rows - (int)blockIdx.x * kRowsPerBlock);
+  t.live = t.node < k;
+  return t;
+}
+
+// Stages the block's rows.  Returns whether their entries fit (else they are
+// read from memory) and sets *first to the block's first entry.
+__device__ __forceinline__ bool bnr_stage(BnrStage& S, int r0, int nr, const int64_t* __restrict__ rp,
+                                          const int* __restrict__ ri,
+                                          const double* __restrict__ rx, int* first) {
+  const int p0 = (int)__ldg(rp + r0);
+  *first = p0;
+  if ((int)threadIdx.x <= nr) S.off[threadIdx.x] = (int)__ldg(rp + r0 + threadIdx.x) - p0;
+  __syncthreads();
+  const int cnt = S.off[nr];
+  if (cnt > kStageCap) return false;
+  for (int q = threadIdx.x; q < cnt; q += kBnrThreads) {
+    S.idx[q] = __ldg(ri + p0 + q);
+    S.val[q] = __ldg(rx + p0 + q);
+  }
+  __syncthreads();
+  return true;
+}
+
+// Row r of the block times the nodes' columns of X, the entries added in
+// storage order, kB gathers in flight.
+template <int V>
+__device__ __forceinline__ Lanes<V> bnr_row(const BnrStage& S, bool staged, int r, int k,
+                                            const int* __restrict__ ri,
+                                            const double* __restrict__ rx,
+                                            const double* __restrict__ Xc) {
+  constexpr int kB = 4;
+  Lanes<V> a;
+#pragma unroll
+  for (int e = 0; e < V; ++e) a.v[e] = 0.0;
+  const int* const idx = staged ? S.idx : ri;
+  const double* const val = staged ? S.val : rx;
+  int q = S.off[r];
+  const int end = S.off[r + 1];
+  for (; q + kB <= end; q += kB) {
+    Lanes<V> x[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) x[u] = Lanes<V>::load(Xc + (long long)idx[q + u] * k);
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const double v = val[q + u];
+#pragma unroll
+      for (int e = 0; e < V; ++e) a.v[e] = add(a.v[e], mul(v, x[u].v[e]));
+    }
+  }
+  if (q < end) {                      // the last 1 .. kB - 1 entries, in flight together
+    Lanes<V> x[kB - 1];
+#pragma unroll
+    for (int u = 0; u < kB - 1; ++u)
+      if (q + u < end) x[u] = Lanes<V>::load(Xc + (long long)idx[q + u] * k);
+#pragma unroll
+    for (int u = 0; u < kB - 1; ++u)
+      if (q + u < end) {
+        const double v = val[q + u];
+#pragma unroll
+        for (int e = 0; e < V; ++e) a.v[e] = add(a.v[e], mul(v, x[u].v[e]));
+      }
+  }
+  return a;
+}
+
+// The block's sums per node from the rows' terms; NS sums.
+template <int V, int NS>
+__device__ __forceinline__ void bnr_sums(BnrStage& S, const BnrTile<V>& t, int k, int pstride,
+                                         int part_block, double* __restrict__ part) {
+  const int tile = t.tile;
+  __syncthreads();                    // the rows' terms are in place
+  for (int w = threadIdx.x; w < 8 * tile; w += kBnrThreads) {
+    const int ph = w / tile, j = w - ph * tile;
+    double a[NS] = {};
+    for (int r = ph; r < t.nr; r += 8) {
+#pragma unroll
+      for (int c = 0; c < NS; ++c) a[c] = add(a[c], S.term[c][r * tile + j]);
+    }
+    // rows ph + 8 j are this thread's alone: its sum may replace the first
+#pragma unroll
+    for (int c = 0; c < NS; ++c) S.term[c][ph * tile + j] = a[c];
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < tile; j += kBnrThreads) {
+    const int node = (int)blockIdx.y * tile + j;
+    if (node >= k) continue;
+    double* out = part + ((long long)node * pstride + part_block) * 2;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      double a = 0.0;
+      if (c < NS) {
+        a = S.term[c][j];
+        for (int y = 1; y < 8; ++y) a = add(a, S.term[c][y * tile + j]);
+      }
+      out[c] = a;
+    }
+  }
+}
+
+// A taken trial is not stored: the next step recomputes it.  pend[j] says
+// that node j's last trial was taken, and eta_prev[j] is the step size that
+// trial used.  The next primal and dual steps read X, AtY, Y and AX anyway;
+// for a pending node they first redo the trial from them with the same
+// operations, which gives the same bits, and store it as the current
+// iterate together with the reference's other updates on acceptance,
+// AtY += AtdY and AX += AdX (bnr.py:262-265).  Nothing is copied, and one
+// buffer per iterate suffices.
+
+// For a node with a taken trial, AtdY = A^T dY (of that trial) and the update;
+// then Xn = clip(X - tau (c + AtY), L, U), dX = Xn - X (bnr.py:233-236), and the
+// node's sum of dX dX over the block's columns.
+template <int V>
+__global__ void __launch_bounds__(kBnrThreads, 2) bnr_cols(
+    int n, int k, int txs, int mblocks, int pstride, const int64_t* __restrict__ cp,
+    const int* __restrict__ ci, const double* __restrict__ cx, const double* __restrict__ c,
+    const double* __restrict__ eta, const double* __restrict__ eta_prev,
+    const double* __restrict__ omega, const int* __restrict__ pend, double* __restrict__ X,
+    double* __restrict__ AtY, const double* __restrict__ dY, const double* __restrict__ L,
+    const double* __restrict__ U, double* __restrict__ dX, double* __restrict__ part) {
+  __shared__ BnrStage S;
+  const BnrTile<V> t = bnr_tile<V>(n, k, txs);
+  const int r0 = blockIdx.x * kRowsPerBlock;
+  grid_dep_release();
+  int first;
+  const bool staged = bnr_stage(S, r0, t.nr, cp, ci, cx, &first);
+  grid_dep_wait();
+  if (t.live) {
+    double tau[V], tau_prev[V];
+    bool taken[V], any = false;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const double om = omega[t.node + e];
+      tau[e] = eta[t.node + e] / om;
+      tau_prev[e] = eta_prev[t.node + e] / om;
+      taken[e] = pend[t.node + e] != 0;
+      any |= taken[e];
+    }
+    for (int r = t.y; r < t.nr; r += t.ty) {
+      const long long g = (long long)(r0 + r) * k + t.node;
+      const double cr = __ldg(c + r0 + r);
+      const Lanes<V> lo = Lanes<V>::load(L + g), hi = Lanes<V>::load(U + g);
+      Lanes<V> x = Lanes<V>::load(X + g), aty = Lanes<V>::load(AtY + g), d;
+      if (any) {
+        const Lanes<V> atdy = bnr_row<V>(S, staged, r, k, ci + first, cx + first, dY + t.node);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (taken[e]) {
+            x.v[e] = clipd(sub(x.v[e], mul(tau_prev[e], add(cr, aty.v[e]))), lo.v[e], hi.v[e]);
+            aty.v[e] = add(aty.v[e], atdy.v[e]);
+          }
+        x.store(X + g);
+        aty.store(AtY + g);
+      }
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const double xn = clipd(sub(x.v[e], mul(tau[e], add(cr, aty.v[e]))), lo.v[e], hi.v[e]);
+        d.v[e] = sub(xn, x.v[e]);
+        S.term[0][r * t.tile + t.x * V + e] = mul(d.v[e], d.v[e]);
+      }
+      d.store(dX + g);
+    }
+  }
+  bnr_sums<V, 1>(S, t, k, pstride, mblocks + blockIdx.x, part);
+}
+
+// The dual trial of a node with step sigma (bnr.py:238-242).
+__device__ __forceinline__ double dual_trial(double y, double ax, double adx, double sigma,
+                                             double lo, double hi) {
+  const double w = add(y, mul(sigma, add(ax, mul(2.0, adx))));
+  return sub(w, mul(sigma, clipd(w / sigma, lo, hi)));
+}
+
+// AdX = A dX; W = Y + sigma (AX + 2 AdX); Yn = W - sigma clip(W / sigma, rl, ru);
+// dY = Yn - Y (bnr.py:238-242), and the node's sums of dY AdX and dY dY over
+// the block's rows.  AdX_prev is the previous step's A dX, which the redone
+// trial uses.
+template <int V>
+__global__ void __launch_bounds__(kBnrThreads, 2) bnr_rows(
+    int m, int k, int txs, int pstride, const int64_t* __restrict__ rp, const int* __restrict__ ri,
+    const double* __restrict__ rx, const double* __restrict__ rl, const double* __restrict__ ru,
+    const double* __restrict__ eta, const double* __restrict__ eta_prev,
+    const double* __restrict__ omega, const int* __restrict__ pend, double* __restrict__ Y,
+    double* __restrict__ AX, const double* __restrict__ AdX_prev, const double* __restrict__ dX,
+    double* __restrict__ AdX, double* __restrict__ dY, double* __restrict__ part) {
+  __shared__ BnrStage S;
+  const BnrTile<V> t = bnr_tile<V>(m, k, txs);
+  const int r0 = blockIdx.x * kRowsPerBlock;
+  grid_dep_release();
+  int first;
+  const bool staged = bnr_stage(S, r0, t.nr, rp, ri, rx, &first);
+  grid_dep_wait();
+  if (t.live) {
+    double sigma[V], sigma_prev[V];
+    bool taken[V], any = false;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const double om = omega[t.node + e];
+      sigma[e] = eta[t.node + e] * om;
+      sigma_prev[e] = eta_prev[t.node + e] * om;
+      taken[e] = pend[t.node + e] != 0;
+      any |= taken[e];
+    }
+    for (int r = t.y; r < t.nr; r += t.ty) {
+      const long long g = (long long)(r0 + r) * k + t.node;
+      const double lo = __ldg(rl + r0 + r), hi = __ldg(ru + r0 + r);
+      Lanes<V> y = Lanes<V>::load(Y + g), ax = Lanes<V>::load(AX + g), d, prev;
+      if (any) prev = Lanes<V>::load(AdX_prev + g);
+      const Lanes<V> adx = bnr_row<V>(S, staged, r, k, ri + first, rx + first, dX + t.node);
+      adx.store(AdX + g);
+      if (any) {
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+          if (taken[e]) {
+            y.v[e] = dual_trial(y.v[e], ax.v[e], prev.v[e], sigma_prev[e], lo, hi);
+            ax.v[e] = add(ax.v[e], prev.v[e]);
+          }
+        y.store(Y + g);
+        ax.store(AX + g);
+      }
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        d.v[e] = sub(dual_trial(y.v[e], ax.v[e], adx.v[e], sigma[e], lo, hi), y.v[e]);
+        S.term[0][r * t.tile + t.x * V + e] = mul(d.v[e], adx.v[e]);
+        S.term[1][r * t.tile + t.x * V + e] = mul(d.v[e], d.v[e]);
+      }
+      d.store(dY + g);
+    }
+  }
+  bnr_sums<V, 2>(S, t, k, pstride, blockIdx.x, part);
+}
+
+// ---- the steps alone, for wide batches ------------------------------------------
+//
+// With many rows times nodes the products run faster as kernels of their own,
+// one row and two nodes per thread (bnr_spmm): see fused_shape.  Block (32, 8)
+// with threadIdx.x the node within a 32-node tile; same sums, same order.
 __device__ __forceinline__ void bnr_block_sums(double s0, double s1, int k, int node,
                                                int pstride, int part_block,
                                                double* __restrict__ part) {
@@ -146,15 +427,6 @@ __device__ __forceinline__ void bnr_block_sums(double s0, double s1, int k, int 
   }
 }
 
-// A taken trial is not stored: the next step recomputes it.  pend[j] says
-// that node j's last trial was taken, and eta_prev[j] is the step size that
-// trial used.  The next primal and dual steps read X, AtY, Y and AX anyway;
-// for a pending node they first redo the trial from them with the same
-// operations, which gives the same bits, and store it as the current
-// iterate together with the reference's other updates on acceptance,
-// AtY += AtdY and AX += AdX (bnr.py:262-265).  Nothing is copied, and one
-// buffer per iterate suffices.
-
 // Xn = clip(X - tau (c + AtY), L, U), dX = Xn - X (bnr.py:233-236), and the
 // node's sum of dX dX over the block's rows.
 __global__ void __launch_bounds__(256) bnr_primal(int n, int k, int mblocks, int pstride,
@@ -170,6 +442,7 @@ __global__ void __launch_bounds__(256) bnr_primal(int n, int k, int mblocks, int
                                                   const double* __restrict__ U,
                                                   double* __restrict__ dX,
                                                   double* __restrict__ part) {
+  grid_dep_wait();
   const int node = blockIdx.y * 32 + threadIdx.x;
   double s = 0.0;
   if (node < k) {
@@ -196,13 +469,6 @@ __global__ void __launch_bounds__(256) bnr_primal(int n, int k, int mblocks, int
   bnr_block_sums(s, 0.0, k, node, pstride, mblocks + blockIdx.x, part);
 }
 
-// The dual trial of a node with step sigma (bnr.py:238-242).
-__device__ __forceinline__ double dual_trial(double y, double ax, double adx, double sigma,
-                                             double lo, double hi) {
-  const double w = add(y, mul(sigma, add(ax, mul(2.0, adx))));
-  return sub(w, mul(sigma, clipd(w / sigma, lo, hi)));
-}
-
 // W = Y + sigma (AX + 2 AdX); Yn = W - sigma clip(W / sigma, rl, ru); dY = Yn - Y
 // (bnr.py:238-242), and the node's sums of dY AdX and dY dY over the block's
 // rows.  AdX_prev is the previous step's A dX, which the redone trial uses.
@@ -218,6 +484,7 @@ __global__ void __launch_bounds__(256) bnr_dual(int m, int k, int pstride,
                                                 const double* __restrict__ AdX,
                                                 double* __restrict__ dY,
                                                 double* __restrict__ part) {
+  grid_dep_wait();
   const int node = blockIdx.y * 32 + threadIdx.x;
   double s0 = 0.0, s1 = 0.0;
   if (node < k) {
@@ -277,6 +544,8 @@ __global__ void __launch_bounds__(128) bnr_accept(int k, int mblocks, int nblock
                                                   const double* __restrict__ fac) {
   const int lane = threadIdx.x & 31;
   const int node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  grid_dep_release();
+  grid_dep_wait();
   if (node >= k) return;            // whole warps leave together
   const int pstride = mblocks + nblocks + 1;
   // the three sums, each in warp_blocks_sum's order, in one loop so that the
@@ -287,14 +556,25 @@ __global__ void __launch_bounds__(128) bnr_accept(int k, int mblocks, int nblock
   const double* pn = base + 2 * (long long)mblocks;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
   const int nmax = max(mblocks, nblocks);
-#pragma unroll 4
-  for (int b = lane; b < nmax; b += 32) {
-    if (b < mblocks) {
-      const double2 v = pm[b];
-      s0 = add(s0, v.x);
-      s1 = add(s1, v.y);
+  constexpr int kU = 8;             // blocks per lane in flight, added in order
+  for (int b0 = lane; b0 < nmax; b0 += 32 * kU) {
+    double2 v[kU];
+    double w[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int b = b0 + 32 * u;
+      v[u] = b < mblocks ? pm[b] : make_double2(0.0, 0.0);
+      w[u] = b < nblocks ? pn[2 * b] : 0.0;
     }
-    if (b < nblocks) s2 = add(s2, pn[2 * b]);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int b = b0 + 32 * u;
+      if (b < mblocks) {
+        s0 = add(s0, v[u].x);
+        s1 = add(s1, v[u].y);
+      }
+      if (b < nblocks) s2 = add(s2, w[u]);
+    }
   }
   double dyadx = __shfl_sync(0xffffffffu, s0, 0), dydy = __shfl_sync(0xffffffffu, s1, 0),
          dxdx = __shfl_sync(0xffffffffu, s2, 0);
@@ -540,31 +820,86 @@ int bnr_upload(T** dst, const T* src, size_t count, int memory, cudaStream_t st)
   return PDLP_OK;
 }
 
+// The fused form for K nodes and `blocks` blocks of 64 rows (both sides), or 0
+// for the split form.  Returns the node tiles and sets the threads along the
+// nodes, 2^txs of V nodes each: four, or eight when four make more blocks than
+// about three per SM.  Beyond five per SM, or with tiles of 32 nodes or more,
+// the split form is as fast or faster (ms per 60 iterations, split against four
+// / eight / sixteen threads: 2,000 x 3,000, 32 nodes 1.45 against 0.76 / 0.96 /
+// 1.30, 128 nodes 1.49 against 1.51 / 1.33 / 1.47; 8,000 x 12,000, 32 nodes 1.58
+// against 1.51 / 1.30 / 1.44, 64 nodes 1.84 against 2.60 / 1.97 / 1.85).
+unsigned fused_shape(int blocks, int K, int V, int* txs) {
+  constexpr long long kThreePerSM = 400, kFivePerSM = 800;
+  auto tiles = [&](int x) { return ((long long)K + (V << x) - 1) / (V << x); };
+  int x = 0;
+  while (x < 2 && tiles(x) > 1) ++x;
+  if (tiles(x) > 1 && blocks * tiles(x) > kThreePerSM) ++x;
+  *txs = x;
+  return blocks * tiles(x) <= kFivePerSM ? (unsigned)tiles(x) : 0u;
+}
+
 // The launches of `iters` iterations for K nodes, on stream s; returns how
 // many kernels it launched.
 long long bnr_enqueue_iterations(pdlp_bnr* b, int K, int iters, cudaStream_t s) {
   const int mblocks = (b->m + kRowsPerBlock - 1) / kRowsPerBlock;
   const int nblocks = (b->n + kRowsPerBlock - 1) / kRowsPerBlock;
-  const dim3 tb(32, 8);
-  const dim3 ngrid(std::max(1, nblocks), (K + 31) / 32), mgrid(std::max(1, mblocks), (K + 31) / 32);
+  const int V = K % 2 == 0 ? 2 : 1;
+  int txs = 0;
+  const unsigned tiles = fused_shape(mblocks + nblocks, K, V, &txs);
+  const bool fused = tiles > 0;
+  const int pstride = mblocks + nblocks + 1;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   long long launches = 0;
+  auto launch = [&](auto kernel, dim3 grid, dim3 block, auto... args) {
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    ++launches;
+  };
+  auto product = [&](int rows, const int64_t* rp, const int* ri, const double* rx,
+                     const double* X, double* Y) {
+    launch(V == 2 ? bnr_spmm<2> : bnr_spmm<1>, dim3((unsigned)blocks_for((long long)rows * (K / V))),
+           dim3(256), rows, K, rp, ri, rx, X, Y);
+  };
   for (int it = 0; it < iters; ++it) {
-    double* adx = (it & 1) ? b->AdX1 : b->AdX0;        // this step's A dX
-    double* adx_prev = (it & 1) ? b->AdX0 : b->AdX1;   // the previous step's
+    double* adx = (it & 1) ? b->AdX1 : b->AdX0;              // this step's A dX
+    const double* adx_prev = (it & 1) ? b->AdX0 : b->AdX1;   // the previous step's
+    const double *c = b->c, *eta = b->eta, *eta_prev = b->eta_prev, *omega = b->omega;
+    const int* pend = b->accept;
     // an empty side has no rows to step and no sums to write
-    if (nblocks > 0)
-      bnr_primal<<<ngrid, tb, 0, s>>>(b->n, K, mblocks, mblocks + nblocks + 1, b->c, b->eta,
-                                      b->eta_prev, b->omega, b->accept, b->X, b->AtY, b->AtdY,
-                                      b->L, b->U, b->dX, b->part);
-    launch_spmm(b->m, K, b->rp, b->ri, b->rx, b->dX, adx, s);
-    if (mblocks > 0)
-      bnr_dual<<<mgrid, tb, 0, s>>>(b->m, K, mblocks + nblocks + 1, b->rl, b->ru, b->eta,
-                                    b->eta_prev, b->omega, b->accept, b->Y, b->AX, adx_prev, adx,
-                                    b->dY, b->part);
-    launch_spmm(b->n, K, b->cp, b->ci, b->cx, b->dY, b->AtdY, s);
-    bnr_accept<<<(K + 3) / 4, 128, 0, s>>>(K, mblocks, nblocks, b->part, b->eta, b->eta_prev,
-                                           b->omega, b->accept, b->fac + 2 * it);
-    launches += 3 + (nblocks > 0) + (mblocks > 0);
+    if (fused) {
+      if (nblocks > 0)
+        launch(V == 2 ? bnr_cols<2> : bnr_cols<1>, dim3((unsigned)nblocks, tiles), dim3(kBnrThreads),
+               b->n, K, txs, mblocks, pstride, (const int64_t*)b->cp, (const int*)b->ci,
+               (const double*)b->cx, c, eta, eta_prev, omega, pend, b->X, b->AtY,
+               (const double*)b->dY, (const double*)b->L, (const double*)b->U, b->dX, b->part);
+      if (mblocks > 0)
+        launch(V == 2 ? bnr_rows<2> : bnr_rows<1>, dim3((unsigned)mblocks, tiles), dim3(kBnrThreads),
+               b->m, K, txs, pstride, (const int64_t*)b->rp, (const int*)b->ri,
+               (const double*)b->rx, (const double*)b->rl, (const double*)b->ru, eta, eta_prev,
+               omega, pend, b->Y, b->AX, adx_prev, (const double*)b->dX, adx, b->dY, b->part);
+    } else {
+      const unsigned kt = (unsigned)((K + 31) / 32);
+      if (nblocks > 0)
+        launch(bnr_primal, dim3((unsigned)nblocks, kt), dim3(32, 8), b->n, K, mblocks, pstride,
+               c, eta, eta_prev, omega, pend, b->X, b->AtY, (const double*)b->AtdY,
+               (const double*)b->L, (const double*)b->U, b->dX, b->part);
+      product(b->m, b->rp, b->ri, b->rx, b->dX, adx);
+      if (mblocks > 0)
+        launch(bnr_dual, dim3((unsigned)mblocks, kt), dim3(32, 8), b->m, K, pstride,
+               (const double*)b->rl, (const double*)b->ru, eta, eta_prev, omega, pend, b->Y, b->AX,
+               adx_prev, (const double*)adx, b->dY, b->part);
+      if (it + 1 < iters) product(b->n, b->cp, b->ci, b->cx, b->dY, b->AtdY);
+    }
+    launch(bnr_accept, dim3((unsigned)((K + 3) / 4)), dim3(128), K, mblocks, nblocks,
+           (const double*)b->part, b->eta, b->eta_prev, omega, b->accept,
+           (const double*)(b->fac + 2 * it));
   }
   return launches;
 }
