@@ -479,86 +479,86 @@ int tune_spmv(int m, const int64_t* rp, const int* ri, const T* rx, const T* x, 
   return rc;
 }
 
-// Y = A X, X row-major (ncols, k).  A thread sums V consecutive columns of
-// one row, in storage order (fused multiply-adds); the block's threads are laid
-// out as (columns / V, rows), so the threads of a row read whole 16-byte
-// pieces of the same rows of X.  The product is bound by those gathers, which
-// L2 serves (nnz k 8 bytes, against 8 k (rows + columns) from memory): four
-// entries' gathers are in flight per thread before their adds.
-template <int V>
-struct Cols;
-template <>
-struct Cols<1> {
-  double v[1];
-  __device__ static Cols load(const double* p) { return Cols{{__ldg(p)}}; }
-  __device__ void store(double* p) const { *p = v[0]; }
-};
-template <>
-struct Cols<2> {
-  double v[2];
-  __device__ static Cols load(const double* p) {
-    const double2 t = __ldg(reinterpret_cast<const double2*>(p));
-    return Cols{{t.x, t.y}};
-  }
-  __device__ void store(double* p) const { *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]); }
-};
-
-template <int V>
-__global__ void __launch_bounds__(kT, 8) spmm_kernel(int m, int k, int col0,
-                                                     const int64_t* __restrict__ rp,
-                                                     const int* __restrict__ ri,
-                                                     const double* __restrict__ rx,
-                                                     const double* __restrict__ X,
-                                                     double* __restrict__ Y) {
-  constexpr int kBatch = 4 / V;
+// Y = A X, X row-major (ncols, k), each row's entries added in storage order by
+// fused multiply-adds.
+//
+// Two columns per thread, where 16-byte pieces fit every row of X and Y: the
+// block's threads are laid out over (columns / 2, rows).  The product is bound by
+// the gathers of X, which L2 serves (nnz k 8 bytes, against 8 k (rows +
+// columns) from memory); two entries' gathers are in flight per thread before
+// their adds, eight blocks per SM.  20,000 x 30,000, 8 entries per column, us at
+// 64 / 160 columns: 18.9 / 48.8 with one column per thread, 14.9 / 37.4 with two.
+__global__ void __launch_bounds__(kT, 8) spmm_pairs_kernel(int m, int k, int col0,
+                                                           const int64_t* __restrict__ rp,
+                                                           const int* __restrict__ ri,
+                                                           const double* __restrict__ rx,
+                                                           const double* __restrict__ X,
+                                                           double* __restrict__ Y) {
+  constexpr int kBatch = 2;
   const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-  const int col = col0 + ((int)blockIdx.y * blockDim.x + threadIdx.x) * V;
+  const int col = col0 + ((int)blockIdx.y * blockDim.x + threadIdx.x) * 2;
   if (row >= m || col >= k) return;
   const double* Xc = X + col;
+  auto gather = [&](long long p) {
+    return __ldg(reinterpret_cast<const double2*>(Xc + (long long)__ldg(ri + p) * k));
+  };
   long long p = __ldg(rp + row);
   const long long end = __ldg(rp + row + 1);
-  double acc[V];
-#pragma unroll
-  for (int e = 0; e < V; ++e) acc[e] = 0.0;
+  double2 acc = make_double2(0.0, 0.0);
   for (; p + kBatch <= end; p += kBatch) {
     double v[kBatch];
-    Cols<V> x[kBatch];
+    double2 x[kBatch];
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
       v[u] = __ldg(rx + p + u);
-      x[u] = Cols<V>::load(Xc + (long long)__ldg(ri + p + u) * k);
+      x[u] = gather(p + u);
     }
 #pragma unroll
-    for (int u = 0; u < kBatch; ++u)
-#pragma unroll
-      for (int e = 0; e < V; ++e) acc[e] = fma(v[u], x[u].v[e], acc[e]);
+    for (int u = 0; u < kBatch; ++u) {
+      acc.x = fma(v[u], x[u].x, acc.x);
+      acc.y = fma(v[u], x[u].y, acc.y);
+    }
   }
   for (; p < end; ++p) {
     const double v = __ldg(rx + p);
-    const Cols<V> x = Cols<V>::load(Xc + (long long)__ldg(ri + p) * k);
-#pragma unroll
-    for (int e = 0; e < V; ++e) acc[e] = fma(v, x.v[e], acc[e]);
+    const double2 x = gather(p);
+    acc.x = fma(v, x.x, acc.x);
+    acc.y = fma(v, x.y, acc.y);
   }
-  Cols<V> out;
-#pragma unroll
-  for (int e = 0; e < V; ++e) out.v[e] = acc[e];
-  out.store(Y + row * k + col);
+  *reinterpret_cast<double2*>(Y + row * k + col) = acc;
 }
 
-// The threads of a block over (columns / V, rows): X's columns in equal parts
-// of at most 32 threads, so that narrow X wastes no lanes, and as many rows as
-// fill the block.
-template <int V>
-void launch_spmm(int m, int k, const int64_t* rp, const int* ri, const double* rx,
-                 const double* X, double* Y, cudaStream_t st) {
+// The block's threads over (columns / 2, rows): X's columns in equal parts of at
+// most 32 threads, so that narrow X wastes no lanes, and as many rows as fill
+// the block.
+void launch_spmm_pairs(int m, int k, const int64_t* rp, const int* ri, const double* rx,
+                       const double* X, double* Y, cudaStream_t st) {
   constexpr int kMaxParts = 65535;
-  const int cols = (k + V - 1) / V, parts = (cols + 31) / 32;
+  const int cols = k / 2, parts = (cols + 31) / 32;
   const int tx = (cols + parts - 1) / parts, ty = kT / tx;
   for (int p0 = 0; p0 < parts; p0 += kMaxParts) {
     const dim3 grid((unsigned)(((long long)m + ty - 1) / ty), (unsigned)std::min(parts - p0, kMaxParts));
-    spmm_kernel<V><<<grid, dim3(tx, ty), 0, st>>>(m, k, p0 * tx * V, rp, ri, rx, X, Y);
+    spmm_pairs_kernel<<<grid, dim3(tx, ty), 0, st>>>(m, k, p0 * tx * 2, rp, ri, rx, X, Y);
     count_launches(1);
   }
+}
+
+// Any k and alignment: one thread per (row, column of X), pairs laid out flat
+// over the threads (38,512 rows, 133 columns: 80 us; 88 with the layout above at
+// one column per thread, 88 to 102 with two to eight gathers in flight).
+__global__ void __launch_bounds__(kT) spmm_kernel(int m, int k, const int64_t* __restrict__ rp,
+                                                  const int* __restrict__ ri,
+                                                  const double* __restrict__ rx,
+                                                  const double* __restrict__ X,
+                                                  double* __restrict__ Y) {
+  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long row = g / k;
+  const int col = (int)(g - row * k);
+  if (row >= m) return;
+  double acc = 0.0;
+  const int64_t p0 = rp[row], p1 = rp[row + 1];
+  for (int64_t p = p0; p < p1; ++p) acc += rx[p] * X[(long long)ri[p] * k + col];
+  Y[row * k + col] = acc;
 }
 
 __global__ void primal_step_kernel(int n, double* xnew, const double* x, const double* c,
@@ -905,11 +905,15 @@ int pdlp_spmm_f64(int32_t m, int32_t k, const int64_t* rp, const int32_t* ri,
   if (m < 0 || k < 0) return fail(PDLP_ERR_ARG, "negative size");
   if (m == 0 || k == 0) return PDLP_OK;
   if (!rp || !ri || !rx || !X || !Y) return fail(PDLP_ERR_ARG, "NULL pointer");
+  const long long blocks = ((long long)m * k + kT - 1) / kT;
   // 16-byte pieces where every row of X and Y starts on one
-  if (k % 2 == 0 && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0)
-    launch_spmm<2>(m, k, rp, ri, rx, X, Y, (cudaStream_t)stream);
-  else
-    launch_spmm<1>(m, k, rp, ri, rx, X, Y, (cudaStream_t)stream);
+  if (k % 2 == 0 && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0) {
+    launch_spmm_pairs(m, k, rp, ri, rx, X, Y, (cudaStream_t)stream);
+  } else {
+    if (blocks > (1LL << 31) - 1) return fail(PDLP_ERR_ARG, "m k too large for an odd k");
+    spmm_kernel<<<(unsigned)blocks, kT, 0, (cudaStream_t)stream>>>(m, k, rp, ri, rx, X, Y);
+    count_launches(1);
+  }
   PDLP_CUDA(cudaGetLastError());
   return PDLP_OK;
 }
