@@ -20,7 +20,8 @@ REPO = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpdlp_b200.so")
 SOURCES = ["engine.cu", "kernels.cu", "spmv_plan.cu", "bnr.cu", "crossover.cu"]
-HEADERS = ["common.cuh", "engine.cuh", "engine_device.cuh", "engine_passes.cuh"]
+HEADERS = ["common.cuh", "engine.cuh", "engine_device.cuh", "engine_passes.cuh",
+           "engine_resident.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

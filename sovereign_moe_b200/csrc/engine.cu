@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "engine_passes.cuh"
+#include "engine_resident.cuh"
 
 namespace pdlp {
 
@@ -95,7 +96,7 @@ __device__ int grid_barrier(Control* ctl, unsigned* counter, unsigned target,
 // no counters, no finisher, no state read.  Alone, in us per iteration with
 // checks and set-up: a 3 x 5 LP 16.2 -> 13.0, 230 x 2,025 20.4 -> 17.9.
 __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
-  WarpSmem* ws = reinterpret_cast<WarpSmem*>(g_smem);
+  WarpSmem* ws = block_warps();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSmem& W = ws[warp];
   if (threadIdx.x == 0) block_flags()[1] = 0;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
 
 // One pass over all tiles of one side; kernel boundaries are the barriers.
 __global__ void __launch_bounds__(kBlock, 3) engine_pass(EngineArgs A, int side) {
-  WarpSmem* ws = reinterpret_cast<WarpSmem*>(g_smem);
+  WarpSmem* ws = block_warps();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSmem& W = ws[warp];
   if (lane == 0) {
@@ -550,6 +551,7 @@ struct Slot {
   std::vector<double> rtw, ctw;   // work estimate per tile
   double bytes_per_iter = 0.0;
   double expected_iters = 0.0;    // the caller's scheduling hint (0: none)
+  int cluster = 0;            // smallest cluster whose shared memory holds it (0: none)
 };
 
 }  // namespace
@@ -621,6 +623,15 @@ struct pdlp_batch {
   pdlp_tuning force{};
   int force_blocks = 0;                // tuning runs: the one team's block count (0: free)
   int withhold_candidate = -1;         // last block of the first multi-block team
+  // clusters: the running LPs that fit one, and the launch's table of them
+  int max_cluster = 0;                 // largest cluster the device runs (0: none are used)
+  std::vector<int> resident;           // slots, at the last rebuild
+  ResidentLP* h_res = nullptr;         // pinned / device, one per slot
+  ResidentLP* d_res = nullptr;
+  int* h_res_steps = nullptr;          // pinned / device: steps each one ran
+  int* d_res_steps = nullptr;
+  cudaStream_t res_streams[5] = {};    // one per cluster size
+  cudaEvent_t res_events[6] = {};      // ready, then one per cluster size
 };
 
 namespace pdlp {
@@ -784,6 +795,69 @@ static double expected_left(const pdlp_batch* b, int s) {
   return -1.0;
 }
 
+// A launch of `count` clusters of `size` CTAs of the resident engine.
+static void res_config(int size, int count, cudaStream_t st, cudaLaunchConfig_t* cfg,
+                       cudaLaunchAttribute* attr) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3((unsigned)(size * count));
+  cfg->blockDim = dim3(kResThreads);
+  cfg->dynamicSmemBytes = kResSmem;
+  cfg->stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)size;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+
+// The largest cluster of a resident kernel that the device can run.
+static int largest_cluster(ResidentKernel kernel) {
+  for (int size = kResMaxCluster; size >= 1; size /= 2) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    res_config(size, 1, nullptr, &cfg, &attr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0) return size;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
+// The largest share of one side's tiles over the CTAs of a cluster.
+static ResShare res_share(const std::vector<Tile>& tiles, int size) {
+  ResShare s{0, 0, 0};
+  for (int q = 0; q < size; ++q) {
+    const int a = res_first((int)tiles.size(), q, size), z = res_first((int)tiles.size(), q + 1, size);
+    if (z <= a) continue;
+    const Tile &ta = tiles[a], &tz = tiles[z - 1];
+    s.tiles = std::max(s.tiles, z - a);
+    s.rows = std::max(s.rows, tz.end - ta.begin);
+    s.nnz = std::max(s.nnz, tz.p0 + tz.cnt - ta.p0);
+  }
+  return s;
+}
+
+static bool res_fits(const Slot& sl, int size) {
+  const ResLayout l = res_layout(sl.m, sl.n, (int)(sl.rt.size() + sl.ct.size()),
+                                 res_share(sl.rt, size), res_share(sl.ct, size), sl.inst.f32 ? 4 : 8);
+  return l.bytes <= kResSmem;
+}
+
+// The smallest cluster that holds the LP (engine_resident.cuh), or 0: 16-bit
+// indices, no row long enough to be a tile of its own, and the engine free to
+// choose where it runs (a tuning run or the withheld-arrival hook wants the
+// team engine, the infeasibility test short launches).
+static int smallest_cluster(const pdlp_batch* b, const Slot& sl) {
+  if (b->max_cluster < 1 || b->force_set || b->cfg.test_withhold_arrival || sl.detect) return 0;
+  if (sl.m < 1 || sl.n < 1 || sl.m > 65535 || sl.n > 65535) return 0;
+  for (const Tile& t : sl.rt) if (t.heavy) return 0;
+  for (const Tile& t : sl.ct) if (t.heavy) return 0;
+  for (int size = 1; size <= b->max_cluster; size *= 2)
+    if (res_fits(sl, size)) return size;
+  return 0;
+}
+
 // The most blocks an instance can use: a warp's tile gathers 512 scattered
 // doubles, and the warps of an SM share its load units, so two tiles a block
 // on twice the SMs finish a pass sooner than one per warp (10,000 x 40,000 in
@@ -892,12 +966,18 @@ static int rebuild(pdlp_batch* b) {
   // where every running slot's tiles and reduction groups go in the launch's
   // lists: row-side groups first, then column-side groups (64 consecutive
   // tiles of a slot per group)
-  std::vector<int> run;                       // running slots, in tile order
-  for (size_t s = 0; s < b->slots.size(); ++s)
-    if (b->slots[s].used && b->slots[s].running) run.push_back((int)s);
+  // the slots the team engine steps come first, those stepped by clusters last
+  std::vector<int> all;                       // running slots, in tile order
+  for (int side = 0; side < 2; ++side)
+    for (size_t s = 0; s < b->slots.size(); ++s)
+      if (b->slots[s].used && b->slots[s].running && (b->slots[s].cluster > 0) == (side == 1))
+        all.push_back((int)s);
+  std::vector<int> run;                       // those of the team engine
+  b->resident.clear();
+  for (int s : all) (b->slots[s].cluster > 0 ? b->resident : run).push_back(s);
   auto ngroups = [](size_t tiles) { return (int)((tiles + kGroupTiles - 1) / kGroupTiles); };
   int nrt = 0, nct = 0, nrg = 0, ncg = 0;
-  for (int s : run) {
+  for (int s : all) {
     Slot& sl = b->slots[s];
     sl.inst.rt_begin = nrt;
     nrt += (int)sl.rt.size();
@@ -909,7 +989,13 @@ static int rebuild(pdlp_batch* b) {
     nrg += ngroups(sl.rt.size());
     sl.inst.rg_end = nrg;
   }
+  int team_nrt = 0, team_nct = 0;             // the team engine's tiles
   for (int s : run) {
+    team_nrt = b->slots[s].inst.rt_end;
+    team_nct = b->slots[s].inst.ct_end;
+  }
+  for (int s : b->resident) b->slots[s].inst.team = kMaxTeams;
+  for (int s : all) {
     Slot& sl = b->slots[s];
     sl.inst.cg_begin = nrg + ncg;
     ncg += ngroups(sl.ct.size());
@@ -926,16 +1012,21 @@ static int rebuild(pdlp_batch* b) {
   // per warp tile ranges, then the team arrays: block_team[G], team_blocks[T],
   // team_first[T], team_inst[T]
   std::vector<int> rwr, cwr, teams;
-  if (tblocks.empty()) {
+  if (run.empty()) {
+    b->grid = 0;
+    b->n_teams = 0;
+    b->withhold_candidate = -1;
+    b->team_running.clear();
+  } else if (tblocks.empty()) {
     std::vector<double> rw, cw;                 // one team splits every running tile
-    rw.reserve(nrt);
-    cw.reserve(nct);
+    rw.reserve(team_nrt);
+    cw.reserve(team_nct);
     for (int s : run) {
       const Slot& sl = b->slots[s];
       rw.insert(rw.end(), sl.rtw.begin(), sl.rtw.end());
       cw.insert(cw.end(), sl.ctw.begin(), sl.ctw.end());
     }
-    const int want = (std::max(b->n_rtiles, b->n_ctiles) + kTilesPerBlock - 1) / kTilesPerBlock;
+    const int want = (std::max(team_nrt, team_nct) + kTilesPerBlock - 1) / kTilesPerBlock;
     int G = std::max(1, std::min(max_blocks, want));
     if (b->force_blocks > 0) G = std::min(G, b->force_blocks);
     b->grid = G;
@@ -975,8 +1066,8 @@ static int rebuild(pdlp_batch* b) {
         cwr.push_back(c0 + pc[q]);
       }
     }
-    rwr.push_back(b->n_rtiles);
-    cwr.push_back(b->n_ctiles);
+    rwr.push_back(team_nrt);
+    cwr.push_back(team_nct);
     for (int k = 0; k < T; ++k) teams.push_back(tblocks[k]);
     for (int k = 0; k < T; ++k) teams.push_back(first[k]);
     for (int k = 0; k < T; ++k) teams.push_back(run[k]);
@@ -1018,7 +1109,7 @@ static int rebuild(pdlp_batch* b) {
   Tile* sct = reinterpret_cast<Tile*>(b->h_stage + up16(b_rt));
   int2* sgr = reinterpret_cast<int2*>(b->h_stage + up16(b_rt) + up16(b_ct));
   Inst* sin = reinterpret_cast<Inst*>(b->h_stage + up16(b_rt) + up16(b_ct) + up16(b_gr));
-  for (int s : run) {
+  for (int s : all) {
     const Slot& sl = b->slots[s];
     const Inst& I = sl.inst;
     for (size_t k = 0; k < sl.rt.size(); ++k) {
@@ -1504,6 +1595,95 @@ static int admit_complete(pdlp_batch* b, Pending& pd, int herr) {
 // the end.  codes[i] receives each LP's code and slots[i] its slot (-1 when
 // refused); the return value is the first failure's code (its message in
 // pdlp_last_error) or PDLP_OK.
+// Launches the resident engine for every running slot that has steps left and
+// fits a cluster, each cluster size on a stream of its own; the batch's stream
+// waits for them.  Slots get the smallest cluster that holds them, doubled as
+// long as all of them still fit the device side by side.
+static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
+  *count = 0;
+  if (b->resident.empty()) return PDLP_OK;
+  if (!b->h_res) {
+    const size_t n = b->slots.size();
+    PDLP_CUDA(cudaMallocHost((void**)&b->h_res, sizeof(ResidentLP) * n));
+    PDLP_CUDA(cudaMallocHost((void**)&b->h_res_steps, sizeof(int) * n));
+    PDLP_CUDA(cudaMalloc((void**)&b->d_res, sizeof(ResidentLP) * n));
+    PDLP_CUDA(cudaMalloc((void**)&b->d_res_steps, sizeof(int) * n));
+  }
+  // growing stops at 8 SMs: 16 gained nothing on LPs that fit 2 (230 x 2,025: 8.6
+  // us per iteration on 4 SMs, 8.4 on 8, 8.3 on 16)
+  constexpr int kGrowTo = 8;
+  long long sms = 0;
+  for (int s : b->resident) sms += b->slots[s].cluster;
+  int grow = 1;
+  while (grow < kGrowTo && sms * grow * 2 <= b->sms - b->sms / 8) grow *= 2;
+  std::vector<int> by_size[5];
+  for (int s : b->resident) {
+    if (b->steps_left[s] <= 0) continue;
+    int k = 0, size = b->slots[s].cluster;
+    while (size * 2 <= std::min(kGrowTo, b->max_cluster) && size < b->slots[s].cluster * grow) size *= 2;
+    while ((1 << k) < size) ++k;
+    by_size[k].push_back(s);
+  }
+  std::vector<int> order;
+  for (int k = 4; k >= 0; --k) {
+    // a launch runs one precision; within it the largest first, so that the
+    // last clusters to start are short
+    std::stable_sort(by_size[k].begin(), by_size[k].end(), [&](int x, int y) {
+      const Slot &sx = b->slots[x], &sy = b->slots[y];
+      return sx.inst.f32 != sy.inst.f32 ? sx.inst.f32 > sy.inst.f32 : sx.nnz > sy.nnz;
+    });
+    for (int s : by_size[k]) {
+      ResidentLP& q = b->h_res[order.size()];
+      q.inst = s;
+      q.budget = (int)std::min<long long>(b->steps_left[s], 1 << 30);
+      q.r = res_share(b->slots[s].rt, 1 << k);
+      q.c = res_share(b->slots[s].ct, 1 << k);
+      order.push_back(s);
+    }
+  }
+  *count = (int)order.size();
+  if (order.empty()) return PDLP_OK;
+  cudaStream_t st = b->stream;
+  PDLP_CUDA(cudaMemcpyAsync(b->d_res, b->h_res, sizeof(ResidentLP) * order.size(), cudaMemcpyHostToDevice, st));
+  // one size: on the batch's stream; several: side by side on streams of
+  // their own, between two points of the batch's stream
+  int sizes = 0;
+  for (const auto& v : by_size) sizes += !v.empty();
+  if (sizes > 1) {
+    if (!b->res_events[5]) {
+      for (cudaEvent_t& e : b->res_events) PDLP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      for (cudaStream_t& q : b->res_streams) PDLP_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+    }
+    PDLP_CUDA(cudaEventRecord(b->res_events[5], st));
+  }
+  size_t first = 0;
+  for (int k = 4; k >= 0; --k) {
+    const size_t n = by_size[k].size();
+    if (n == 0) continue;
+    const cudaStream_t q = sizes > 1 ? b->res_streams[k] : st;
+    if (sizes > 1) PDLP_CUDA(cudaStreamWaitEvent(q, b->res_events[5], 0));
+    for (size_t a = 0; a < n;) {
+      const int f32 = b->slots[by_size[k][a]].inst.f32;
+      size_t z = a;
+      while (z < n && b->slots[by_size[k][z]].inst.f32 == f32) ++z;
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr;
+      res_config(1 << k, (int)(z - a), q, &cfg, &attr);
+      PDLP_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel(f32 != 0), A,
+                                   (const ResidentLP*)(b->d_res + first + a),
+                                   b->d_res_steps + first + a));
+      count_launches(1);
+      a = z;
+    }
+    if (sizes > 1) {
+      PDLP_CUDA(cudaEventRecord(b->res_events[k], b->res_streams[k]));
+      PDLP_CUDA(cudaStreamWaitEvent(st, b->res_events[k], 0));
+    }
+    first += n;
+  }
+  return PDLP_OK;
+}
+
 static int admit_many(pdlp_batch* b, int count, const pdlp_problem_desc* const* probs,
                       const pdlp_params* const* params, int32_t* slots, int32_t* codes) {
   if (!b) return fail(PDLP_ERR_ARG, "NULL batch");
@@ -1600,6 +1780,7 @@ static int admit_many(pdlp_batch* b, int count, const pdlp_problem_desc* const* 
     Slot& S = b->slots[pd[i].slot];
     plan_tiles(pd[i].rp, probs[i]->m, pd[i].slot, pd[i].tile_rows, pd[i].tile_nnz, S.rt, S.rtw);
     plan_tiles(pd[i].cp, probs[i]->n, pd[i].slot, pd[i].tile_rows, pd[i].tile_nnz, S.ct, S.ctw);
+    S.cluster = smallest_cluster(b, S);
   });
   PDLP_CUDA(cudaStreamSynchronize(st));    // the initial states have left h_init
   for (int i = 0; i < count; ++i) {
@@ -1701,6 +1882,17 @@ int pdlp_batch_create(const pdlp_batch_config* cfg, void* stream, pdlp_batch** o
                                                           kBlock, kSmemBytes)) != cudaSuccess)
     return bail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
   if (!coop || b->coop_blocks_per_sm < 1) b->cfg.persistent = 0;
+  if (b->cfg.persistent) {
+    b->max_cluster = kResMaxCluster;
+    for (int f32 = 0; f32 < 2; ++f32) {
+      const ResidentKernel k = resident_kernel(f32 != 0);
+      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem)) != cudaSuccess)
+        return bail(e, "cudaFuncSetAttribute");
+      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
+        return bail(e, "cudaFuncSetAttribute");
+      b->max_cluster = std::min(b->max_cluster, largest_cluster(k));
+    }
+  }
   if ((e = cudaMalloc(&b->d_inst, sizeof(Inst) * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = cudaMalloc(&b->d_state, sizeof(State) * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = cudaMalloc(&b->d_counters, sizeof(unsigned) * 2 * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
@@ -1753,6 +1945,12 @@ int pdlp_batch_destroy(pdlp_batch* b) {
   if (b->h_tasks) cudaFreeHost(b->h_tasks);
   cudaFree(b->d_pieces);
   cudaFree(b->d_tasks);
+  if (b->h_res) cudaFreeHost(b->h_res);
+  if (b->h_res_steps) cudaFreeHost(b->h_res_steps);
+  cudaFree(b->d_res);
+  cudaFree(b->d_res_steps);
+  for (cudaStream_t q : b->res_streams) if (q) cudaStreamDestroy(q);
+  for (cudaEvent_t q : b->res_events) if (q) cudaEventDestroy(q);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   delete b;
@@ -1831,6 +2029,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     A.withhold_block = (b->cfg.persistent && b->cfg.test_withhold_arrival) ? b->withhold_candidate : -1;
     b->h_ctl->bar_count = 0; b->h_ctl->bar_gen = 0; b->h_ctl->active = b->n_running;
     b->h_ctl->error = 0; b->h_ctl->error_where = 0; b->h_ctl->stop = 0; b->h_ctl->idle = 0;
+    b->h_ctl->team_active[kMaxTeams] = (int)b->resident.size();
     for (int t = 0; t < kMaxTeams; ++t) {
       b->h_ctl->team_bar[t] = 0;
       b->h_ctl->team_active[t] = t < (int)b->team_running.size() ? b->team_running[t] : 0;
@@ -1839,17 +2038,21 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     }
     for (size_t s = 0; s < b->slots.size(); ++s) {
       const Slot& sl = b->slots[s];
-      if (!sl.used || !sl.running) continue;
+      if (!sl.used || !sl.running || sl.cluster > 0) continue;
       const int t = b->n_teams > 1 ? sl.inst.team : 0;
       b->h_ctl->team_budget[t] = (int)std::min<int64_t>(b->steps_left[s], kChunk);
     }
     PDLP_CUDA(cudaMemcpyAsync(b->d_ctl, b->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, st));
     PDLP_CUDA(cudaEventRecord(b->ev0, st));
+    int n_res = 0;
     if (b->cfg.persistent) {
-      void* args[] = {&A};
-      PDLP_CUDA(cudaLaunchCooperativeKernel((void*)engine_persistent, dim3(b->grid), dim3(kBlock),
-                                            args, kSmemBytes, st));
-      count_launches(1);
+      if ((rc = launch_resident(b, A, &n_res))) return rc;
+      if (b->grid > 0) {
+        void* args[] = {&A};
+        PDLP_CUDA(cudaLaunchCooperativeKernel((void*)engine_persistent, dim3(b->grid), dim3(kBlock),
+                                              args, kSmemBytes, st));
+        count_launches(1);
+      }
     } else {
       if (b->graph_stale || !b->graph || b->graph_chunk != chunk) {
         if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
@@ -1880,6 +2083,9 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     PDLP_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, st));
     PDLP_CUDA(cudaMemcpyAsync(b->h_state, b->d_state, sizeof(State) * b->slots.size(),
                               cudaMemcpyDeviceToHost, st));
+    if (n_res > 0)
+      PDLP_CUDA(cudaMemcpyAsync(b->h_res_steps, b->d_res_steps, sizeof(int) * n_res,
+                                cudaMemcpyDeviceToHost, st));
     PDLP_CUDA(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, b->ev0, b->ev1);
@@ -1925,11 +2131,13 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
       return fail(b->h_ctl->error, "engine: a bounded device wait timed out; the batch was stopped");
     }
     int running = 0;
+    for (int q = 0; q < n_res; ++q) b->steps_left[b->h_res[q].inst] -= b->h_res_steps[q];
     for (size_t s = 0; s < b->slots.size(); ++s) {
       Slot& sl = b->slots[s];
       if (!sl.used || !sl.running) continue;
-      b->steps_left[s] -= b->cfg.persistent ? b->h_ctl->team_steps[b->n_teams > 1 ? sl.inst.team : 0]
-                                            : chunk;
+      if (sl.cluster == 0)
+        b->steps_left[s] -= b->cfg.persistent ? b->h_ctl->team_steps[b->n_teams > 1 ? sl.inst.team : 0]
+                                              : chunk;
       const State& hs = b->h_state[s];
       long long d = hs.iters_done - b->iters_before[s];
       b->iters_before[s] = hs.iters_done;

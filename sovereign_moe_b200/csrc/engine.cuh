@@ -169,7 +169,8 @@ struct Control {
   unsigned int idle;        // blocks of teams whose instances are all done
   unsigned int pad;
   unsigned int team_bar[kMaxTeams];   // each team's barrier arrival counter
-  int team_active[kMaxTeams];         // each team's instances still running
+  int team_active[kMaxTeams + 1];     // each team's instances still running (the last: those
+                                      // stepped by clusters)
   int team_budget[kMaxTeams];         // steps each team may run in this launch (host)
   int team_steps[kMaxTeams];          // steps each team completed (its leader, at exit)
 };

@@ -144,15 +144,16 @@ struct BulkPhase {
   bool flush = true;
 };
 
-// The block's shared memory: the warps' areas, then three words: the barrier's
-// verdict, whether a wait or check inside the block failed (the block then
-// leaves at its next barrier), and whether the team has instances running.
+// The block's shared memory: three words -- the barrier's verdict, whether a
+// wait or check inside the block failed (the block then leaves at its next
+// barrier), and whether the team has instances running -- then the warps'
+// areas.
 extern __shared__ __align__(16) unsigned char g_smem[];
-constexpr size_t kSmemBytes = sizeof(WarpSmem) * kWarps + 16;
+constexpr size_t kSmemBytes = 16 + sizeof(WarpSmem) * kWarps;
 
-__device__ __forceinline__ volatile int* block_flags() {
-  return reinterpret_cast<volatile int*>(g_smem + sizeof(WarpSmem) * kWarps);
-}
+__device__ __forceinline__ volatile int* block_flags() { return reinterpret_cast<volatile int*>(g_smem); }
+
+__device__ __forceinline__ WarpSmem* block_warps() { return reinterpret_cast<WarpSmem*>(g_smem + 16); }
 
 __device__ __forceinline__ void block_fail() { block_flags()[1] = 1; }
 

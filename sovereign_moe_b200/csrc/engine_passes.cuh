@@ -52,6 +52,19 @@ __device__ __forceinline__ double merit(double omega, double p, double d, double
   return sqrt((omega * p) * (omega * p) + (d / omega) * (d / omega) + g * g);
 }
 
+// The test of a trial step and the next step size (pdlp.py:340-381).
+__device__ __forceinline__ bool step_test(double eta, double omega, double dxdx, double dyadx,
+                                          double dydy, long long attempts, double* eta_new) {
+  const double interaction = fabs(dyadx);
+  const double movement = 0.5 * (omega * dxdx + dydy / omega);
+  *eta_new = eta;
+  if (movement == 0.0) return true;
+  const double eta_limit = interaction > 0.0 ? movement / interaction : INFINITY;
+  const double t = (double)(attempts + 1);
+  *eta_new = fmax(fmin((1.0 - pow(t, -0.3)) * eta_limit, (1.0 + pow(t, -0.6)) * eta), 1e-14);
+  return eta <= eta_limit;
+}
+
 // ---- teams of one LP: the warps' copies of its scheduling fields -------------
 
 __device__ __forceinline__ void team_load(TeamCopy& c, const State* S, int lane) {
@@ -246,25 +259,11 @@ __device__ void r_finish(const EngineArgs& A, const Inst& I, State* S, int rmode
     case R_APPLY: S->rhs_orig = red[0]; S->bn2 = red[1]; break;
     case R_POWER: if (S->power_round == 1) S->p0 = red[0]; break;
     case R_TRIAL: {
-      // adaptive step (pdlp.py:340-381)
       S->attempts += 1;
       S->trials += 1;
-      const double eta = S->eta, omega = S->omega;
-      const double interaction = fabs(red[0]);
-      const double movement = 0.5 * (omega * S->dxdx + red[1] / omega);
-      bool accepted = false;
-      double eta_new = eta;
-      if (movement == 0.0) {
-        accepted = true;
-      } else {
-        const double eta_limit = interaction > 0.0 ? movement / interaction : INFINITY;
-        const double t = (double)(S->attempts + 1);
-        const double eta_next = fmax(fmin((1.0 - pow(t, -0.3)) * eta_limit,
-                                          (1.0 + pow(t, -0.6)) * eta), 1e-14);
-        if (eta <= eta_limit) accepted = true;
-        else S->rejected += 1;
-        eta_new = eta_next;
-      }
+      double eta_new;
+      const bool accepted = step_test(S->eta, S->omega, S->dxdx, red[0], red[1], S->attempts, &eta_new);
+      if (!accepted) S->rejected += 1;
       S->eta = eta_new;
       if (accepted) {
         S->trials = 0;
