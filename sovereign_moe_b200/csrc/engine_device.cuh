@@ -176,11 +176,13 @@ struct Ops {
   }
 };
 
-// Warp-wide reduction of kNP slots with a fixed xor tree; every lane ends
-// with the result.
-__device__ __forceinline__ void warp_reduce(double* v, Ops ops) {
+// Warp-wide reduction of the first `n` of kNP slots with a fixed xor tree;
+// every lane ends with the result.  (A pass uses 1 to 7 slots; a slot costs
+// five dependent shuffles of a double.)
+__device__ __forceinline__ void warp_reduce(double* v, Ops ops, int n) {
 #pragma unroll
   for (int s = 0; s < kNP; ++s) {
+    if (s >= n) break;
     const int op = ops.op(s);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v[s] = combine(v[s], __shfl_xor_sync(kFull, v[s], off), op);
@@ -196,15 +198,18 @@ __device__ __forceinline__ void warp_reduce(double* v, Ops ops) {
 // storage order, then a xor butterfly; L == 1 is the storage-order sum).
 // Heavy tile (one row longer than a normal tile holds): the 32 lanes stride
 // over the row, then a xor butterfly.  Either way the order depends only on
-// the row and L.  term(p, rhs) returns the factors value[p], x_rhs[index[p]].
+// the row and L.  term(p, j, rhs) returns the factors value[p], x_rhs[j] for the
+// column j = index[p]; sidx[q] is the index of the tile's entry q (staged by
+// the caller: the gathers do not wait for it), idx the array it comes from.
 struct Factors {
   double a, x;
 };
 constexpr int kHeavyLoads = 8;
 
 template <int NR, class F>
-__device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const int* tptr, int L,
-                                          F term, WarpSmem& W, int lane) {
+__device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const int* tptr,
+                                          const int* idx, const int* sidx, int L, F term,
+                                          WarpSmem& W, int lane) {
   if (t.heavy) {
     const int p0 = ld_ro(ptr + t.begin), p1 = ld_ro(ptr + t.begin + 1);
     double a0 = 0.0, a1 = 0.0;
@@ -218,8 +223,9 @@ __device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const i
       Factors f[kU], g[NR == 2 ? kU : 1];
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
-        f[u] = term(p + 32 * u, 0);
-        if (NR == 2) g[u] = term(p + 32 * u, 1);
+        const int j = ld_ro(idx + p + 32 * u);
+        f[u] = term(p + 32 * u, j, 0);
+        if (NR == 2) g[u] = term(p + 32 * u, j, 1);
       }
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
@@ -229,10 +235,11 @@ __device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const i
     }
 #pragma unroll 1
     for (; p < p1; p += 32) {
-      const Factors f = term(p, 0);
+      const int j = ld_ro(idx + p);
+      const Factors f = term(p, j, 0);
       a0 = fma(f.a, f.x, a0);
       if (NR == 2) {
-        const Factors g = term(p, 1);
+        const Factors g = term(p, j, 1);
         a1 = fma(g.a, g.x, a1);
       }
     }
@@ -258,7 +265,7 @@ __device__ __forceinline__ void warp_spmv(const Tile& t, const int* ptr, const i
         const int q = q0 + u * 32 + lane;
         v[u] = 0.0;
         if (q < cnt) {
-          const Factors f = term(p0 + q, rhs);
+          const Factors f = term(p0 + q, sidx[q], rhs);
           v[u] = f.a * f.x;
         }
       }

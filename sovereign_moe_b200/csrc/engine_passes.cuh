@@ -127,7 +127,8 @@ __device__ void team_flush(const TeamCopy& c, State* S) {
 // pass uses the counter one way only.
 __device__ __forceinline__ bool warp_finish(const EngineArgs& A, const Tile& t, int side,
                                             int g_first, int g_last, int n_tiles, bool need_red,
-                                            Ops ops, double* res, int lane, BulkPhase& ph) {
+                                            Ops ops, int slots, double* res, int lane,
+                                            BulkPhase& ph) {
   ph.pend += 1;
   if (!ph.flush) return false;
   const unsigned done = ph.pend;
@@ -159,9 +160,10 @@ __device__ __forceinline__ bool warp_finish(const EngineArgs& A, const Tile& t, 
     for (int s = 0; s < kNP; ++s) v[s] = identity_of(ops.op(s));
     for (int tt = gt.x + lane; tt < gt.y; tt += 32) {
 #pragma unroll
-      for (int s = 0; s < kNP; ++s) v[s] = combine(v[s], ld_mut(tp + (size_t)tt * kNP + s), ops.op(s));
+      for (int s = 0; s < kNP; ++s)
+        if (s < slots) v[s] = combine(v[s], ld_mut(tp + (size_t)tt * kNP + s), ops.op(s));
     }
-    warp_reduce(v, ops);
+    warp_reduce(v, ops, slots);
     if (lane == 0 && g_last - g_first > 1) {
 #pragma unroll
       for (int s = 0; s < kNP; ++s) A.gpartials[(size_t)g * kNP + s] = v[s];
@@ -188,9 +190,10 @@ __device__ __forceinline__ bool warp_finish(const EngineArgs& A, const Tile& t, 
     for (int s = 0; s < kNP; ++s) v[s] = identity_of(ops.op(s));
     for (int gg = g_first + lane; gg < g_last; gg += 32) {
 #pragma unroll
-      for (int s = 0; s < kNP; ++s) v[s] = combine(v[s], ld_mut(A.gpartials + (size_t)gg * kNP + s), ops.op(s));
+      for (int s = 0; s < kNP; ++s)
+        if (s < slots) v[s] = combine(v[s], ld_mut(A.gpartials + (size_t)gg * kNP + s), ops.op(s));
     }
-    warp_reduce(v, ops);
+    warp_reduce(v, ops, slots);
 #pragma unroll
     for (int s = 0; s < kNP; ++s) res[s] = v[s];
   }
@@ -488,11 +491,12 @@ __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst
 #endif
 #undef HOT_STAMP
   const bool need_red = rmode == R_TRIAL;
+  constexpr int slots = 2;
   // a team of one LP retires a commit in its copies (TeamCopy)
   const bool need_fin = need_red || (commit && team == nullptr);
   Ops ops;
   if (need_red) {
-    warp_reduce(acc, ops);
+    warp_reduce(acc, ops, slots);
     if (lane == 0) {
 #pragma unroll
       for (int s = 0; s < kNP; ++s) A.partials[(size_t)ti * kNP + s] = acc[s];
@@ -500,8 +504,8 @@ __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst
   }
   if (!need_fin) return;
   double res[kNP];
-  if (warp_finish(A, t, 0, I.rg_begin, I.rg_end, I.rt_end - I.rt_begin, need_red, ops, res,
-                  lane, ph)) {
+  if (warp_finish(A, t, 0, I.rg_begin, I.rg_end, I.rt_end - I.rt_begin, need_red, ops, slots,
+                  res, lane, ph)) {
     if (lane == 0) {
       if (team) team_flush(*team, S);
       r_finish(A, I, S, rmode, res);
@@ -574,17 +578,18 @@ __device__ void hot_ctile(const EngineArgs& A, const Tile& t, int ti, const Inst
   }
   if (quiet) return;
   const bool need_red = cprimal == P_TRIAL;
+  constexpr int slots = 1;
   Ops ops;
   if (need_red) {
-    warp_reduce(acc, ops);
+    warp_reduce(acc, ops, slots);
     if (lane == 0) {
 #pragma unroll
       for (int s = 0; s < kNP; ++s) A.partials[(size_t)(A.n_rtiles + ti) * kNP + s] = acc[s];
     }
   }
   double res[kNP];
-  if (warp_finish(A, t, 1, I.cg_begin, I.cg_end, I.ct_end - I.ct_begin, need_red, ops, res,
-                  lane, ph)) {
+  if (warp_finish(A, t, 1, I.cg_begin, I.cg_end, I.ct_end - I.ct_begin, need_red, ops, slots,
+                  res, lane, ph)) {
     if (lane == 0) {
       if (team) team_flush(*team, S);
       c_finish(A, I, S, cmode, res);
@@ -635,6 +640,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
   if (!t.heavy && !bulk_wait(A, &W.bar[0], ph.m)) return;
   __syncwarp();
   const int* tptr = W.sptr + offp;
+  const int* sidx = W.sidx + offi;
   if (!t.heavy && !tile_ptrs_ok(A, t, tptr, lane)) return;
 
   const int L = I.lanes_r;
@@ -746,14 +752,13 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double scale = ld_mut(&S->power_scale);
       const double* v = I.xbar;                    // A^T A power vector
       const double* rx = I.rx;
-      auto term = [&](int p, int rhs) {
-        const int j = ld_ro(ri + p);
+      auto term = [&](int p, int j, int rhs) {
         const double a = ld_mut(rx + p);
         if (rhs == 0) return Factors{a, scale != 0.0 ? ld_mut(v + j) / scale : 0.0};
         return Factors{a, ld_mut(I.x + j)};
       };
-      if (round == 1) warp_spmv<2>(t, rp, tptr, L, term, W, lane);
-      else warp_spmv<1>(t, rp, tptr, L, term, W, lane);
+      if (round == 1) warp_spmv<2>(t, rp, tptr, ri, sidx, L, term, W, lane);
+      else warp_spmv<1>(t, rp, tptr, ri, sidx, L, term, W, lane);
       ops.maxmask = 1u;
       for (int r = t.begin + lane; r < rend; r += 32) {
         const int li = r - t.begin;
@@ -770,8 +775,8 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       // backend.py:260-279: ax += adx; w = y + sigma (ax + adx); prox; dy
       const double* rx = I.rx;
       const double* dxv = I.dx;
-      warp_spmv<1>(t, rp, tptr, L, [&](int p, int) {
-        return Factors{ld_mut(rx + p), ld_mut(dxv + ld_ro(ri + p))};
+      warp_spmv<1>(t, rp, tptr, ri, sidx, L, [&](int p, int j, int) {
+        return Factors{ld_mut(rx + p), ld_mut(dxv + j)};
       }, W, lane);
       for (int r = t.begin + lane; r < rend; r += 32) {
         do_commit(r);
@@ -792,8 +797,8 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       // pdlp.py:347-356: adx = A dx; ax_bar = ax + 2 adx; dual_step; dy; dots
       const double* rx = I.rx;
       const double* dxv = I.dx;
-      warp_spmv<1>(t, rp, tptr, L, [&](int p, int) {
-        return Factors{ld_mut(rx + p), ld_mut(dxv + ld_ro(ri + p))};
+      warp_spmv<1>(t, rp, tptr, ri, sidx, L, [&](int p, int j, int) {
+        return Factors{ld_mut(rx + p), ld_mut(dxv + j)};
       }, W, lane);
       for (int r = t.begin + lane; r < rend; r += 32) {
         do_commit(r);
@@ -834,8 +839,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* rx = I.rx;
       const double* xb = I.xbar;
       const double* xc = I.x;
-      warp_spmv<2>(t, rp, tptr, L, [&](int p, int rhs) {
-        const int j = ld_ro(ri + p);
+      warp_spmv<2>(t, rp, tptr, ri, sidx, L, [&](int p, int j, int rhs) {
         return Factors{ld_mut(rx + p), ld_mut((rhs == 0 ? xb : xc) + j)};
       }, W, lane);
       ops.maxmask = 7u;
@@ -881,9 +885,11 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
   // pending commit; the other modes reduce and/or advance the state machine.
   const bool need_red = rmode == R_RUIZ || rmode == R_APPLY || rmode == R_POWER ||
                         rmode == R_TRIAL || rmode == R_CHECK_A || rmode == R_CHECK_B;
+  const int slots = rmode == R_CHECK_A ? 5 : rmode == R_CHECK_B ? 3
+                  : rmode == R_APPLY || rmode == R_TRIAL ? 2 : 1;
   const bool need_fin = !(rmode == R_ITER && (!commit || team != nullptr));
   if (need_red) {
-    warp_reduce(acc, ops);
+    warp_reduce(acc, ops, slots);
     if (lane == 0) {
 #pragma unroll
       for (int s = 0; s < kNP; ++s) A.partials[(size_t)ti * kNP + s] = acc[s];
@@ -891,8 +897,8 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
   }
   if (!need_fin) return;
   double res[kNP];
-  if (warp_finish(A, t, 0, I.rg_begin, I.rg_end, I.rt_end - I.rt_begin, need_red, ops, res,
-                  lane, ph)) {
+  if (warp_finish(A, t, 0, I.rg_begin, I.rg_end, I.rt_end - I.rt_begin, need_red, ops, slots,
+                  res, lane, ph)) {
     if (lane == 0) {
       if (team) team_flush(*team, S);
       r_finish(A, I, S, rmode, res);
@@ -1149,6 +1155,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
   if (!t.heavy && !bulk_wait(A, &W.bar[0], ph.m)) return;
   __syncwarp();
   const int* tptr = W.sptr + offp;
+  const int* sidx = W.sidx + offi;
   if (!t.heavy && !tile_ptrs_ok(A, t, tptr, lane)) return;
 
   const int L = I.lanes_c;
@@ -1266,8 +1273,8 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
     case C_POWER: {
       const double* cx = I.cx;
       const double* av = I.ybar;
-      warp_spmv<1>(t, cp, tptr, L, [&](int p, int) {
-        return Factors{ld_mut(cx + p), ld_mut(av + ld_ro(ci + p))};
+      warp_spmv<1>(t, cp, tptr, ci, sidx, L, [&](int p, int i, int) {
+        return Factors{ld_mut(cx + p), ld_mut(av + i)};
       }, W, lane);
       for (int j = t.begin + lane; j < rend; j += 32) {
         const double v = W.s0[j - t.begin];
@@ -1282,8 +1289,8 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const bool xc = xcommit;
       const int kind = cprimal;
       const double* dyv = I.dy;
-      warp_spmv<1>(t, cp, tptr, L, [&](int p, int) {
-        return Factors{ld_mut(cx + p), ld_mut(dyv + ld_ro(ci + p))};
+      warp_spmv<1>(t, cp, tptr, ci, sidx, L, [&](int p, int i, int) {
+        return Factors{ld_mut(cx + p), ld_mut(dyv + i)};
       }, W, lane);
       for (int j = t.begin + lane; j < rend; j += 32) {
         const double xv = xc ? ld_mut(I.xnew + j) : ld_mut(I.x + j);
@@ -1327,8 +1334,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const double* cx = I.cx;
       const double* yb = I.ybar;
       const double* yc = I.y;
-      warp_spmv<2>(t, cp, tptr, L, [&](int p, int rhs) {
-        const int i = ld_ro(ci + p);
+      warp_spmv<2>(t, cp, tptr, ci, sidx, L, [&](int p, int i, int rhs) {
         return Factors{ld_mut(cx + p), ld_mut((rhs == 0 ? yb : yc) + i)};
       }, W, lane);
       const double s = ld_mut(&S->s_obj);
@@ -1372,8 +1378,8 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
       const bool avg = ld_mut(&S->final_src) != 0;
       const double* ysrc = avg ? I.ybar : I.y;
       const double* cx = I.cx;
-      warp_spmv<1>(t, cp, tptr, L, [&](int p, int) {
-        return Factors{ld_mut(cx + p), ld_mut(ysrc + ld_ro(ci + p))};
+      warp_spmv<1>(t, cp, tptr, ci, sidx, L, [&](int p, int i, int) {
+        return Factors{ld_mut(cx + p), ld_mut(ysrc + i)};
       }, W, lane);
       const double s = ld_mut(&S->s_obj);
       const double dsign = I.sense == 1 ? 1.0 : -1.0;
@@ -1396,8 +1402,10 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
   const bool need_red = trial || cmode == C_RUIZ || cmode == C_APPLY || cmode == C_SETUP0 ||
                         cmode == C_POWER || cmode == C_CHECK_A || cmode == C_CHECK_B ||
                         cmode == C_FINAL;
+  const int slots = cmode == C_CHECK_B ? 7 : cmode == C_CHECK_A ? 6 : cmode == C_SETUP0 ? 5
+                  : cmode == C_APPLY ? 3 : 1;
   if (need_red) {
-    warp_reduce(acc, ops);
+    warp_reduce(acc, ops, slots);
     if (lane == 0) {
 #pragma unroll
       for (int s = 0; s < kNP; ++s)
@@ -1405,8 +1413,8 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
     }
   }
   double res[kNP];
-  if (warp_finish(A, t, 1, I.cg_begin, I.cg_end, I.ct_end - I.ct_begin, need_red, ops, res,
-                  lane, ph)) {
+  if (warp_finish(A, t, 1, I.cg_begin, I.cg_end, I.ct_end - I.ct_begin, need_red, ops, slots,
+                  res, lane, ph)) {
     if (lane == 0) {
       if (team) team_flush(*team, S);
       c_finish(A, I, S, cmode, res);

@@ -48,8 +48,8 @@ constexpr int kResMaxCluster = 16;
 // copy of the scheduling fields per warp for the generic passes.
 struct __align__(16) ResHeader {
   int flags[4];            // block_flags()
-  int failed;              // rank 0's view of the launch's error word
-  int pad[3];
+  int failed[2];           // rank 0's view of the launch's error word, by generic step
+  int pad[2];
   Inst inst;
   State st;
   TeamCopy team[kResWarps];
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
     const int* src = reinterpret_cast<const int*>(A.inst + lp.inst);
     int* dst = reinterpret_cast<int*>(&H.inst);
     for (int i = threadIdx.x; i < (int)(sizeof(Inst) / sizeof(int)); i += kResThreads) dst[i] = src[i];
-    if (threadIdx.x == 0) H.failed = 0;
+    if (threadIdx.x == 0) H.failed[0] = H.failed[1] = 0;
     __syncthreads();
   }
   const Inst& I = H.inst;
@@ -722,6 +722,8 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
   const int r0 = I.rt_begin + res_first(nrt, gw, nw), r1 = I.rt_begin + res_first(nrt, gw + 1, nw);
   const int c0 = I.ct_begin + res_first(nct, gw, nw), c1 = I.ct_begin + res_first(nct, gw + 1, nw);
   int step = 0;
+  int turn = 0;
+  bool started = false;                // every CTA has met a barrier of this kernel
   while (step < lp.budget) {
     team_load(C, S, lane);
     if (C.rmode == R_NONE && C.cmode == C_NONE) break;           // the LP is done
@@ -731,8 +733,15 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
       continue;
     }
     // one step of the generic passes
+    // (the descriptor comes from the CTA's copy: W shares its memory with the
+    // resident data)
+    {
+      const int* src = reinterpret_cast<const int*>(&H.inst);
+      int* dst = reinterpret_cast<int*>(&W.inst);
+      for (int i = lane; i < (int)(sizeof(Inst) / sizeof(int)); i += 32) dst[i] = src[i];
+    }
     if (lane == 0) {
-      W.inst_id = -1;
+      W.inst_id = lp.inst;
       mbar_init(&W.bar[0]);
       mbar_init(&W.bar[1]);
       mbar_init_fence();
@@ -749,6 +758,7 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
         process_rtile(A, cur, t, W, lane, pc, ph, &C);
       }
       cluster_sync_global(lane);
+      started = true;
       team_load(C, S, lane);
     }
     if (C.cmode != C_NONE) {
@@ -759,20 +769,25 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
         ph.flush = t + 1 >= c1 || A.ctiles[t + 1].group != cur.group;
         process_ctile(A, cur, t, W, lane, pc, ph, &C, false);
       }
-      cluster_sync_global(lane);
     }
     __syncwarp();
     if (lane == 0) {
       mbar_inval(&W.bar[0]);
       mbar_inval(&W.bar[1]);
     }
-    // a bounded wait that gave up (here or elsewhere in the launch): every CTA
-    // of the cluster leaves on rank 0's word
-    if (rank == 0 && threadIdx.x == 0)
-      cluster_put(&H.failed, *(volatile int*)&A.ctl->error, size);
-    cluster_sync();
+    // a bounded wait that gave up (in an earlier pass, here or elsewhere in the
+    // launch): every CTA of the cluster leaves on rank 0's word, written once
+    // every CTA is known to run
+    if (rank == 0 && threadIdx.x == 0) {
+      const int e = *(volatile int*)&A.ctl->error;
+      if (started) cluster_put(&H.failed[turn], e, size);
+    }
+    cluster_sync_global(lane);
+    started = true;
     ++step;
-    if (H.failed != 0) break;
+    // two words in turn: this one is next written after every thread has read it
+    if (H.failed[turn] != 0) break;
+    turn ^= 1;
   }
   if (rank == 0 && threadIdx.x == 0) steps_done[blockIdx.x / size] = step;
   cluster_sync();                // no CTA leaves while a peer may write into it
