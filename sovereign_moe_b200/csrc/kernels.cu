@@ -488,13 +488,14 @@ int tune_spmv(int m, const int64_t* rp, const int* ri, const T* rx, const T* x, 
 // columns) from memory); two entries' gathers are in flight per thread before
 // their adds, eight blocks per SM.  20,000 x 30,000, 8 entries per column, us at
 // 64 / 160 columns: 18.9 / 48.8 with one column per thread, 14.9 / 37.4 with two.
-__global__ void __launch_bounds__(kT, 8) spmm_pairs_kernel(int m, int k, int col0,
-                                                           const int64_t* __restrict__ rp,
-                                                           const int* __restrict__ ri,
-                                                           const double* __restrict__ rx,
-                                                           const double* __restrict__ X,
-                                                           double* __restrict__ Y) {
-  constexpr int kBatch = 2;
+// A product that leaves half the chip's threads without work is bound by the
+// chain of a row's gathers instead and keeps eight in flight (kSpmmFew).
+constexpr long long kSpmmFew = 148 * 1024;
+
+template <int kBatch>
+__global__ void __launch_bounds__(kT, kBatch == 2 ? 8 : 2) spmm_pairs_kernel(
+    int m, int k, int col0, const int64_t* __restrict__ rp, const int* __restrict__ ri,
+    const double* __restrict__ rx, const double* __restrict__ X, double* __restrict__ Y) {
   const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
   const int col = col0 + ((int)blockIdx.y * blockDim.x + threadIdx.x) * 2;
   if (row >= m || col >= k) return;
@@ -519,11 +520,23 @@ __global__ void __launch_bounds__(kT, 8) spmm_pairs_kernel(int m, int k, int col
       acc.y = fma(v[u], x[u].y, acc.y);
     }
   }
-  for (; p < end; ++p) {
-    const double v = __ldg(rx + p);
-    const double2 x = gather(p);
-    acc.x = fma(v, x.x, acc.x);
-    acc.y = fma(v, x.y, acc.y);
+  if (p < end) {                      // the last 1 .. kBatch - 1 entries, in flight together
+    double v[kBatch - 1];
+    double2 x[kBatch - 1];
+#pragma unroll
+    for (int u = 0; u < kBatch - 1; ++u) {
+      if (p + u < end) {
+        v[u] = __ldg(rx + p + u);
+        x[u] = gather(p + u);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch - 1; ++u) {
+      if (p + u < end) {
+        acc.x = fma(v[u], x[u].x, acc.x);
+        acc.y = fma(v[u], x[u].y, acc.y);
+      }
+    }
   }
   *reinterpret_cast<double2*>(Y + row * k + col) = acc;
 }
@@ -538,7 +551,10 @@ void launch_spmm_pairs(int m, int k, const int64_t* rp, const int* ri, const dou
   const int tx = (cols + parts - 1) / parts, ty = kT / tx;
   for (int p0 = 0; p0 < parts; p0 += kMaxParts) {
     const dim3 grid((unsigned)(((long long)m + ty - 1) / ty), (unsigned)std::min(parts - p0, kMaxParts));
-    spmm_pairs_kernel<<<grid, dim3(tx, ty), 0, st>>>(m, k, p0 * tx * 2, rp, ri, rx, X, Y);
+    if ((long long)m * cols <= kSpmmFew)
+      spmm_pairs_kernel<8><<<grid, dim3(tx, ty), 0, st>>>(m, k, p0 * tx * 2, rp, ri, rx, X, Y);
+    else
+      spmm_pairs_kernel<2><<<grid, dim3(tx, ty), 0, st>>>(m, k, p0 * tx * 2, rp, ri, rx, X, Y);
     count_launches(1);
   }
 }

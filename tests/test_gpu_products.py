@@ -138,3 +138,22 @@ def test_chained_products_keep_stream_order(bk, dtype):
     for _ in range(3):
         got = chain(False)
         assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("m,k", [(2_501, 120), (2_501, 122), (1, 2), (40_000, 6), (40_000, 8)])
+def test_spmm_gathers_in_flight(bk, m, k):
+    """Both sides of the line (148 * 1024 pairs of columns) between eight and two
+    gathers in flight, rows of 0 to 20 entries: the same bits as the flat form,
+    which unaligned blocks take."""
+    import torch
+    rng = np.random.default_rng([m, k])
+    n = 300
+    rp, ri, rx = _csr(rng, rng.integers(0, 21, m), n)
+    args = (bk.pointer(rp), bk.index(ri), bk.to_device(rx))
+    X = bk.to_device(rng.standard_normal((n, k)))
+    a = bk.empty((m, k))
+    bk.spmm(*args, X, a, m, k)
+    Xs, Ys = bk.empty(n * k + 1)[1:], bk.empty(m * k + 1)[1:]
+    Xs.copy_(X.reshape(-1))
+    bk.spmm(*args, Xs, Ys, m, k)
+    assert torch.equal(a.reshape(-1), Ys)
