@@ -22,7 +22,7 @@ import numpy as np
 
 from . import _lib
 from .pdlp import (PDLPParams, _check_device, _to_solution, params_struct, problem_desc,
-                   start_with_problem)
+                   reference_start, start_with_problem)
 
 __all__ = ["BatchEngine"]
 
@@ -111,14 +111,28 @@ class BatchEngine:
         descs = (_lib.ProblemDesc * count)()
         prms = (_lib.Params * count)()
         keep = []
+        shared = []          # device-resident LPs that start from the reference's vector
         for i, prob in enumerate(probs):
-            d, k = problem_desc(prob)
+            d, k = problem_desc(prob, sync=False)
             p, kv = params_struct(params, int(prob.A.n), power_start=power_start)
-            kv = start_with_problem(d, p, kv)
+            if d.memory == _lib.PDLP_MEM_DEVICE and isinstance(power_start, str):
+                shared.append(i)
+            else:
+                kv = start_with_problem(d, p, kv)
             if hints is not None:
                 p.expected_iterations = float(hints[i])
             descs[i], prms[i] = d, p
             keep.append((k, kv))
+        if shared:
+            # one copy of the start on the device: shorter ones are its prefixes
+            import torch
+            start = torch.tensor(reference_start(max(descs[i].n for i in shared)), device="cuda")
+            for i in shared:
+                prms[i].power_start = start.data_ptr() if descs[i].n else None
+            keep.append(start)
+        if any(d.memory == _lib.PDLP_MEM_DEVICE for d in descs):
+            import torch
+            torch.cuda.current_stream().synchronize()    # before the engine's stream reads
         slots = np.full(count, -1, dtype=np.int32)
         codes = np.zeros(count, dtype=np.int32)
         self.lib.pdlp_batch_admit_many(self.h, count, descs, prms, slots.ctypes.data,
@@ -199,7 +213,25 @@ class BatchEngine:
         for c in codes:
             _lib.check(c)
         self.run()
-        out = [self.fetch(s) for s in slots]
-        for s in slots:
-            self.retire(s)
+        return self.collect(slots)
+
+    def collect(self, slots):
+        """The finished slots' Solutions, and the slots retired, with two
+        synchronisations in all (``pdlp_batch_collect_many``)."""
+        count = len(slots)
+        meta = [self._meta[s] for s in slots]
+        res = (_lib.Result * count)()
+        xs = [np.empty(int(p.A.n)) for p, _, _, _ in meta]
+        ys = [np.empty(int(p.A.m)) for p, _, _, _ in meta]
+        ds = [np.empty(int(p.A.n)) for p, _, _, _ in meta]
+        hists = [np.empty(5 * max(hcap, 1)) for _, _, hcap, _ in meta]
+        ptrs = [(ctypes.c_void_p * count)(*[a.ctypes.data for a in arrs])
+                for arrs in (xs, ys, ds, hists)]
+        _lib.check(self.lib.pdlp_batch_collect_many(self.h, count, (ctypes.c_int32 * count)(*slots),
+                                                    res, *ptrs, _lib.PDLP_MEM_HOST, 1))
+        now = time.perf_counter()
+        out = []
+        for i, (prob, params, _, t0) in enumerate(meta):
+            out.append(_to_solution(prob, params, res[i], xs[i], ys[i], ds[i], hists[i], now - t0))
+            self._meta.pop(slots[i], None)
         return out

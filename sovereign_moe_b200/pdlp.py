@@ -81,6 +81,28 @@ class PDLPInfo:
     device_seconds: float = 0.0
 
 
+# The reference's power-iteration start, default_rng(0).standard_normal(n)
+# (pdlp.py:142-143): a longer draw begins with every shorter one, so one draw of
+# up to 2^20 elements (8 MB, read-only) serves every n below it.  A draw costs 9
+# ns an element: 6 ms for 600,000 columns, more than the solve of a small LP.
+_START_KEPT = 1 << 20
+_start = np.empty(0)
+
+
+def reference_start(n):
+    """``default_rng(0).standard_normal(n)``, read-only."""
+    global _start
+    have = _start
+    if n > _START_KEPT:
+        return np.random.default_rng(0).standard_normal(n)
+    if n > have.shape[0]:
+        have = np.random.default_rng(0).standard_normal(min(_START_KEPT, 1 << (n - 1).bit_length()))
+        have.flags.writeable = False
+        if have.shape[0] > _start.shape[0]:      # another thread may have drawn more
+            _start = have
+    return have[:n]
+
+
 def _host(a, dtype):
     return np.ascontiguousarray(a, dtype=dtype)
 
@@ -97,10 +119,11 @@ def _numpy(a, dtype=np.float64):
     return np.asarray(a, dtype=dtype)
 
 
-def _device_desc(prob):
+def _device_desc(prob, sync=True):
     """A ``pdlp_problem_desc`` over CUDA tensors: ``prob``'s arrays stay on the
     device (converted to the ABI's types there when needed) and the engine
-    copies them into the slot's arena on the device."""
+    copies them into the slot's arena on the device.  Without ``sync`` the
+    caller synchronises the current stream before the engine reads them."""
     import torch
     A = prob.A
     f64, i32, i64 = torch.float64, torch.int32, torch.int64
@@ -125,11 +148,12 @@ def _device_desc(prob):
     d.obj_offset = float(prob.obj_offset)
     d.sense = -1 if int(prob.sense) == int(ObjSense.MAXIMISE) else 1
     d.memory = _lib.PDLP_MEM_DEVICE
-    torch.cuda.current_stream().synchronize()    # conversions done before the engine's stream reads
+    if sync:
+        torch.cuda.current_stream().synchronize()    # conversions done before the engine's stream reads
     return d, arrs
 
 
-def problem_desc(prob, flip_free=True):
+def problem_desc(prob, flip_free=True, sync=True):
     """A ``pdlp_problem_desc`` over ``prob``'s arrays: host copies, or, when
     the matrix values are a CUDA tensor, the device arrays themselves
     (``_device_desc``).
@@ -138,7 +162,7 @@ def problem_desc(prob, flip_free=True):
     uses ``desc``."""
     A = prob.A
     if _on_device(A.rx):
-        return _device_desc(prob)
+        return _device_desc(prob, sync)
     arrs = dict(
         rp=_host(A.rp, np.int64), ri=_host(A.ri, np.int32), rx=_host(A.rx, np.float64),
         cp=_host(A.cp, np.int64), ci=_host(A.ci, np.int32), cx=_host(A.cx, np.float64),
@@ -192,7 +216,7 @@ def params_struct(params: PDLPParams, n: int, time_used: float = 0.0, history_ca
     p.history_capacity = int(history_capacity)
     keep = None
     if isinstance(power_start, str) and power_start == "reference":
-        keep = np.random.default_rng(0).standard_normal(n)
+        keep = reference_start(n)
     elif power_start is not None:
         keep = np.ascontiguousarray(power_start, dtype=np.float64)
     p.power_start = keep.ctypes.data if keep is not None and keep.size else None
@@ -206,7 +230,7 @@ def start_with_problem(desc, p, keep_v0):
     ``p.power_start`` points there.  Returns what must be kept alive."""
     if desc.memory == _lib.PDLP_MEM_DEVICE and keep_v0 is not None and keep_v0.size:
         import torch
-        keep_v0 = torch.as_tensor(keep_v0, device="cuda")
+        keep_v0 = torch.tensor(keep_v0, device="cuda")
         torch.cuda.current_stream().synchronize()
         p.power_start = keep_v0.data_ptr()
     return keep_v0
