@@ -732,8 +732,12 @@ struct RedPool {
 std::map<int, RedPool> red_pools;   // by device
 
 void red_free(RedSlot& s) {
+  // allowed while a stream captures, as in red_make
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   if (s.partials) cudaFree(s.partials);
   if (s.out) cudaFreeHost(s.out);
+  cudaThreadExchangeStreamCaptureMode(&mode);
   s = RedSlot{};
 }
 
