@@ -552,6 +552,8 @@ struct Slot {
   double bytes_per_iter = 0.0;
   double expected_iters = 0.0;    // the caller's scheduling hint (0: none)
   int cluster = 0;            // smallest cluster whose shared memory holds it (0: none)
+  bool off_chip = false;      // the team engine steps it all the same (kResSteps)
+  bool on_chip() const { return cluster > 0 && !off_chip; }
 };
 
 }  // namespace
@@ -866,8 +868,137 @@ static int smallest_cluster(const pdlp_batch* b, const Slot& sl) {
 // rows: 111, 98 and 96 ms).
 constexpr int kTilesPerBlock = 2;
 
+// The most steps of a launch on chip, alone and with LPs for the team engine.
+// The batch's launches take turns, so LPs on chip keep the team engine's
+// waiting.  One that has used a whole launch while others need the team engine
+// goes on there beside them (both engines give the same bits), until only LPs
+// that fit clusters are left; so a long solve on chip holds nobody up.
+// (It moves only to a team of its own: a team of several LPs steps all of them
+// by one budget.)  256 uneven LPs, a fifth of them too large for a cluster: LPs/s with estimates,
+// ms without, by the steps before an LP moves: 128 550, 442; 256 546, 443; 512
+// 540, 447; 1,024 535, 450; 2,048 530, 456; 4,096 513, 456; 16,384 498, 484.
+// Alone the limit lets LPs that do not all fit the GPU at once take turns too.
+constexpr int kResSteps = 16384, kResStepsBeside = 256;
+
+// Puts every LP back on chip once no running LP needs the team engine.
+static void return_on_chip(pdlp_batch* b) {
+  for (const Slot& sl : b->slots)
+    if (sl.used && sl.running && sl.cluster == 0) return;
+  for (Slot& sl : b->slots) {
+    if (!sl.used || !sl.running || !sl.off_chip) continue;
+    sl.off_chip = false;
+    b->dirty = true;
+  }
+}
+
+// Launches the resident engine for every running slot that has steps left and
+// fits a cluster, each cluster size on a stream of its own; the batch's stream
+// waits for them.  Slots get the smallest cluster that holds them, doubled as
+// long as all of them still fit the device side by side.
+static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
+  *count = 0;
+  if (b->resident.empty()) return PDLP_OK;
+  const size_t slots = b->slots.size();
+  if (!b->h_res) PDLP_CUDA(cudaMallocHost((void**)&b->h_res, sizeof(ResidentLP) * slots));
+  if (!b->h_res_steps) PDLP_CUDA(cudaMallocHost((void**)&b->h_res_steps, sizeof(int) * slots));
+  if (!b->d_res) PDLP_CUDA(cudaMalloc((void**)&b->d_res, sizeof(ResidentLP) * slots));
+  if (!b->d_res_steps) PDLP_CUDA(cudaMalloc((void**)&b->d_res_steps, sizeof(int) * slots));
+  // growing stops at 8 SMs: 16 gained nothing on LPs that fit 2 (230 x 2,025: 8.6
+  // us per iteration on 4 SMs, 8.4 on 8, 8.3 on 16)
+  constexpr int kGrowTo = 8;
+  long long sms = 0;
+  for (int s : b->resident) sms += b->slots[s].cluster;
+  int grow = 1;
+  while (grow < kGrowTo && sms * grow * 2 <= b->sms - b->sms / 8) grow *= 2;
+  std::vector<int> by_size[5];
+  for (int s : b->resident) {
+    if (b->steps_left[s] <= 0) continue;
+    int k = 0, size = b->slots[s].cluster;
+    while (size * 2 <= std::min(kGrowTo, b->max_cluster) && size < b->slots[s].cluster * grow) size *= 2;
+    while ((1 << k) < size) ++k;
+    by_size[k].push_back(s);
+  }
+  const int most = b->grid > 0 ? kResStepsBeside : kResSteps;
+  std::vector<int> order;
+  // A launch runs one precision; within it the longest first, so that the last
+  // clusters to start are short: by the iterations each LP is expected to need
+  // if that is known for all, else by entries.  An iteration on chip costs
+  // nearly the same whatever the entries: 256 uneven LPs with estimates, 204 of
+  // them on chip to their end, ran at 498 LPs/s so, 496 and 491 with iterations
+  // times (entries + 20,000) and times entries, 486 by entries alone.
+  std::vector<double> work(b->slots.size());
+  bool known = true;
+  for (int s : b->resident) {
+    work[s] = expected_left(b, s);
+    known = known && work[s] > 0.0;
+  }
+  if (!known)
+    for (int s : b->resident) work[s] = (double)b->slots[s].nnz;
+  for (int k = 4; k >= 0; --k) {
+    std::stable_sort(by_size[k].begin(), by_size[k].end(), [&](int x, int y) {
+      const Slot &sx = b->slots[x], &sy = b->slots[y];
+      return sx.inst.f32 != sy.inst.f32 ? sx.inst.f32 > sy.inst.f32 : work[x] > work[y];
+    });
+    for (int s : by_size[k]) {
+      ResidentLP& q = b->h_res[order.size()];
+      q.inst = s;
+      q.budget = (int)std::min<long long>(b->steps_left[s], most);
+      q.r = res_share(b->slots[s].rt, 1 << k);
+      q.c = res_share(b->slots[s].ct, 1 << k);
+      order.push_back(s);
+    }
+  }
+  *count = (int)order.size();
+  if (order.empty()) return PDLP_OK;
+  cudaStream_t st = b->stream;
+  PDLP_CUDA(cudaMemcpyAsync(b->d_res, b->h_res, sizeof(ResidentLP) * order.size(), cudaMemcpyHostToDevice, st));
+  // one size: on the batch's stream; several: side by side on streams of
+  // their own, between two points of the batch's stream
+  int sizes = 0;
+  for (const auto& v : by_size) sizes += !v.empty();
+  if (sizes > 1) {
+    for (cudaEvent_t& e : b->res_events)
+      if (!e) PDLP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (cudaStream_t& q : b->res_streams)
+      if (!q) PDLP_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+    PDLP_CUDA(cudaEventRecord(b->res_events[5], st));
+  }
+  size_t first = 0;
+  for (int k = 4; k >= 0; --k) {
+    const size_t n = by_size[k].size();
+    if (n == 0) continue;
+    const cudaStream_t q = sizes > 1 ? b->res_streams[k] : st;
+    if (sizes > 1) PDLP_CUDA(cudaStreamWaitEvent(q, b->res_events[5], 0));
+    for (size_t a = 0; a < n;) {
+      const int f32 = b->slots[by_size[k][a]].inst.f32;
+      size_t z = a;
+      while (z < n && b->slots[by_size[k][z]].inst.f32 == f32) ++z;
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute attr;
+      res_config(1 << k, (int)(z - a), q, &cfg, &attr);
+      PDLP_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel(f32 != 0), A,
+                                   (const ResidentLP*)(b->d_res + first + a),
+                                   b->d_res_steps + first + a));
+      count_launches(1);
+      a = z;
+    }
+    if (sizes > 1) {
+      PDLP_CUDA(cudaEventRecord(b->res_events[k], b->res_streams[k]));
+      PDLP_CUDA(cudaStreamWaitEvent(st, b->res_events[k], 0));
+    }
+    first += n;
+  }
+  return PDLP_OK;
+}
+
+// The most instances that get a team each on `max_blocks` blocks.
+static int most_teams(int max_blocks) {
+  constexpr int kTeamsFrom = 256;
+  return std::min({kTeamsFrom, kMaxTeams, max_blocks});
+}
+
 // The block teams of a persistent launch.  With many running instances one
-// team of blocks steps them all.  With fewer (at most kTeamsFrom), each
+// team of blocks steps them all.  With fewer (at most most_teams), each
 // instance gets its own team, so that no instance waits at a barrier for
 // another's tiles.  Teams get blocks in proportion to each instance's weight,
 // but never more than leave kTilesPerBlock tiles a block: the blocks an instance
@@ -886,10 +1017,8 @@ constexpr int kTilesPerBlock = 2;
 // order, or nothing for one team.
 static std::vector<int> plan_teams(const pdlp_batch* b, const std::vector<int>& run,
                                    int max_blocks) {
-  constexpr int kTeamsFrom = 256;
   std::vector<int> tblocks;
-  if (!b->cfg.persistent || run.size() < 2 ||
-      (int)run.size() > std::min(kTeamsFrom, kMaxTeams) || (int)run.size() > max_blocks)
+  if (!b->cfg.persistent || run.size() < 2 || (int)run.size() > most_teams(max_blocks))
     return tblocks;
   const size_t T = run.size();
   bool hinted = true;
@@ -970,11 +1099,11 @@ static int rebuild(pdlp_batch* b) {
   std::vector<int> all;                       // running slots, in tile order
   for (int side = 0; side < 2; ++side)
     for (size_t s = 0; s < b->slots.size(); ++s)
-      if (b->slots[s].used && b->slots[s].running && (b->slots[s].cluster > 0) == (side == 1))
+      if (b->slots[s].used && b->slots[s].running && b->slots[s].on_chip() == (side == 1))
         all.push_back((int)s);
   std::vector<int> run;                       // those of the team engine
   b->resident.clear();
-  for (int s : all) (b->slots[s].cluster > 0 ? b->resident : run).push_back(s);
+  for (int s : all) (b->slots[s].on_chip() ? b->resident : run).push_back(s);
   auto ngroups = [](size_t tiles) { return (int)((tiles + kGroupTiles - 1) / kGroupTiles); };
   int nrt = 0, nct = 0, nrg = 0, ncg = 0;
   for (int s : all) {
@@ -1595,107 +1724,6 @@ static int admit_complete(pdlp_batch* b, Pending& pd, int herr) {
 // the end.  codes[i] receives each LP's code and slots[i] its slot (-1 when
 // refused); the return value is the first failure's code (its message in
 // pdlp_last_error) or PDLP_OK.
-// Launches the resident engine for every running slot that has steps left and
-// fits a cluster, each cluster size on a stream of its own; the batch's stream
-// waits for them.  Slots get the smallest cluster that holds them, doubled as
-// long as all of them still fit the device side by side.
-static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
-  *count = 0;
-  if (b->resident.empty()) return PDLP_OK;
-  if (!b->h_res) {
-    const size_t n = b->slots.size();
-    PDLP_CUDA(cudaMallocHost((void**)&b->h_res, sizeof(ResidentLP) * n));
-    PDLP_CUDA(cudaMallocHost((void**)&b->h_res_steps, sizeof(int) * n));
-    PDLP_CUDA(cudaMalloc((void**)&b->d_res, sizeof(ResidentLP) * n));
-    PDLP_CUDA(cudaMalloc((void**)&b->d_res_steps, sizeof(int) * n));
-  }
-  // growing stops at 8 SMs: 16 gained nothing on LPs that fit 2 (230 x 2,025: 8.6
-  // us per iteration on 4 SMs, 8.4 on 8, 8.3 on 16)
-  constexpr int kGrowTo = 8;
-  long long sms = 0;
-  for (int s : b->resident) sms += b->slots[s].cluster;
-  int grow = 1;
-  while (grow < kGrowTo && sms * grow * 2 <= b->sms - b->sms / 8) grow *= 2;
-  std::vector<int> by_size[5];
-  for (int s : b->resident) {
-    if (b->steps_left[s] <= 0) continue;
-    int k = 0, size = b->slots[s].cluster;
-    while (size * 2 <= std::min(kGrowTo, b->max_cluster) && size < b->slots[s].cluster * grow) size *= 2;
-    while ((1 << k) < size) ++k;
-    by_size[k].push_back(s);
-  }
-  std::vector<int> order;
-  // A launch runs one precision; within it the longest first, so that the last
-  // clusters to start are short: by the iterations each LP is expected to need
-  // if that is known for all, else by entries.  An iteration on chip costs
-  // nearly the same whatever the entries: 256 uneven LPs with estimates run at
-  // 498 LPs/s so, 496 and 491 with iterations times (entries + 20,000) and times
-  // entries, 486 by entries alone.
-  std::vector<double> work(b->slots.size());
-  bool known = true;
-  for (int s : b->resident) {
-    work[s] = expected_left(b, s);
-    known = known && work[s] > 0.0;
-  }
-  if (!known)
-    for (int s : b->resident) work[s] = (double)b->slots[s].nnz;
-  for (int k = 4; k >= 0; --k) {
-    std::stable_sort(by_size[k].begin(), by_size[k].end(), [&](int x, int y) {
-      const Slot &sx = b->slots[x], &sy = b->slots[y];
-      return sx.inst.f32 != sy.inst.f32 ? sx.inst.f32 > sy.inst.f32 : work[x] > work[y];
-    });
-    for (int s : by_size[k]) {
-      ResidentLP& q = b->h_res[order.size()];
-      q.inst = s;
-      q.budget = (int)std::min<long long>(b->steps_left[s], 1 << 30);
-      q.r = res_share(b->slots[s].rt, 1 << k);
-      q.c = res_share(b->slots[s].ct, 1 << k);
-      order.push_back(s);
-    }
-  }
-  *count = (int)order.size();
-  if (order.empty()) return PDLP_OK;
-  cudaStream_t st = b->stream;
-  PDLP_CUDA(cudaMemcpyAsync(b->d_res, b->h_res, sizeof(ResidentLP) * order.size(), cudaMemcpyHostToDevice, st));
-  // one size: on the batch's stream; several: side by side on streams of
-  // their own, between two points of the batch's stream
-  int sizes = 0;
-  for (const auto& v : by_size) sizes += !v.empty();
-  if (sizes > 1) {
-    if (!b->res_events[5]) {
-      for (cudaEvent_t& e : b->res_events) PDLP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      for (cudaStream_t& q : b->res_streams) PDLP_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-    }
-    PDLP_CUDA(cudaEventRecord(b->res_events[5], st));
-  }
-  size_t first = 0;
-  for (int k = 4; k >= 0; --k) {
-    const size_t n = by_size[k].size();
-    if (n == 0) continue;
-    const cudaStream_t q = sizes > 1 ? b->res_streams[k] : st;
-    if (sizes > 1) PDLP_CUDA(cudaStreamWaitEvent(q, b->res_events[5], 0));
-    for (size_t a = 0; a < n;) {
-      const int f32 = b->slots[by_size[k][a]].inst.f32;
-      size_t z = a;
-      while (z < n && b->slots[by_size[k][z]].inst.f32 == f32) ++z;
-      cudaLaunchConfig_t cfg;
-      cudaLaunchAttribute attr;
-      res_config(1 << k, (int)(z - a), q, &cfg, &attr);
-      PDLP_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel(f32 != 0), A,
-                                   (const ResidentLP*)(b->d_res + first + a),
-                                   b->d_res_steps + first + a));
-      count_launches(1);
-      a = z;
-    }
-    if (sizes > 1) {
-      PDLP_CUDA(cudaEventRecord(b->res_events[k], b->res_streams[k]));
-      PDLP_CUDA(cudaStreamWaitEvent(st, b->res_events[k], 0));
-    }
-    first += n;
-  }
-  return PDLP_OK;
-}
-
 static int admit_many(pdlp_batch* b, int count, const pdlp_problem_desc* const* probs,
                       const pdlp_params* const* params, int32_t* slots, int32_t* codes) {
   if (!b) return fail(PDLP_ERR_ARG, "NULL batch");
@@ -1793,6 +1821,7 @@ static int admit_many(pdlp_batch* b, int count, const pdlp_problem_desc* const* 
     plan_tiles(pd[i].rp, probs[i]->m, pd[i].slot, pd[i].tile_rows, pd[i].tile_nnz, S.rt, S.rtw);
     plan_tiles(pd[i].cp, probs[i]->n, pd[i].slot, pd[i].tile_rows, pd[i].tile_nnz, S.ct, S.ctw);
     S.cluster = smallest_cluster(b, S);
+    S.off_chip = false;
   });
   PDLP_CUDA(cudaStreamSynchronize(st));    // the initial states have left h_init
   for (int i = 0; i < count; ++i) {
@@ -2021,11 +2050,13 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
   for (size_t s = 0; s < b->slots.size(); ++s)
     b->steps_left[s] = (b->slots[s].used && b->slots[s].running) ? std::max<int64_t>(max_steps, 0) : 0;
   double total_ms = 0.0;
+  std::vector<int> moved;             // LPs that leave the chip after this launch
   while (b->n_running > 0) {
     int64_t most = 0;                 // the largest budget left among running LPs
     for (size_t s = 0; s < b->slots.size(); ++s)
       if (b->slots[s].used && b->slots[s].running) most = std::max<int64_t>(most, b->steps_left[s]);
     if (most <= 0) break;
+    return_on_chip(b);
     if (b->dirty && (rc = rebuild(b))) return rc;
     A.rtiles = b->d_rtiles; A.n_rtiles = b->n_rtiles;
     A.ctiles = b->d_ctiles; A.n_ctiles = b->n_ctiles;
@@ -2050,7 +2081,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     }
     for (size_t s = 0; s < b->slots.size(); ++s) {
       const Slot& sl = b->slots[s];
-      if (!sl.used || !sl.running || sl.cluster > 0) continue;
+      if (!sl.used || !sl.running || sl.on_chip()) continue;
       const int t = b->n_teams > 1 ? sl.inst.team : 0;
       b->h_ctl->team_budget[t] = (int)std::min<int64_t>(b->steps_left[s], kChunk);
     }
@@ -2142,12 +2173,16 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
                                          "; the batch was stopped");
       return fail(b->h_ctl->error, "engine: a bounded device wait timed out; the batch was stopped");
     }
-    int running = 0;
-    for (int q = 0; q < n_res; ++q) b->steps_left[b->h_res[q].inst] -= b->h_res_steps[q];
+    int running = 0, teams = 0;         // teams: the team engine's LPs
+    for (int q = 0; q < n_res; ++q) {
+      const int s = b->h_res[q].inst;
+      b->steps_left[s] -= b->h_res_steps[q];
+      if (b->grid > 0 && b->h_res_steps[q] >= kResStepsBeside) moved.push_back(s);
+    }
     for (size_t s = 0; s < b->slots.size(); ++s) {
       Slot& sl = b->slots[s];
       if (!sl.used || !sl.running) continue;
-      if (sl.cluster == 0)
+      if (!sl.on_chip())
         b->steps_left[s] -= b->cfg.persistent ? b->h_ctl->team_steps[b->n_teams > 1 ? sl.inst.team : 0]
                                               : chunk;
       const State& hs = b->h_state[s];
@@ -2158,6 +2193,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
       if (hs.status != PDLP_STATUS_RUNNING) { sl.running = false; b->dirty = true; }
       else {
         ++running;
+        teams += !sl.on_chip();
         if (hs.rmode == R_NONE && hs.cmode == C_NONE) {
           b->broken = true;
           return fail(PDLP_ERR_STATE, "engine: a running LP has no pass scheduled (internal error)");
@@ -2176,6 +2212,14 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
         }
       }
     }
+    for (int s : moved) {
+      Slot& sl = b->slots[s];
+      if (!sl.running || teams >= most_teams(std::max(1, b->sms * b->coop_blocks_per_sm))) continue;
+      sl.off_chip = true;
+      b->dirty = true;
+      ++teams;
+    }
+    moved.clear();
     b->n_running = running;
   }
   b->last_ms = total_ms;

@@ -102,3 +102,40 @@ def test_cancel_and_retire_between_budgets():
         got = eng.fetch(again)
     ref = _bits([probs[1]], _params(), False)[0]
     assert (got.iterations, got.x.tobytes()) == (ref[0], ref[7])
+
+
+@pytest.mark.parametrize("order", [(0, 1, 2), (2, 1, 0)])
+def test_engines_hand_over_to_each_other(order):
+    """LPs that use up a whole launch on chip while another LP needs the team
+    engine go on beside it there, and return on chip when it has finished."""
+    lps = [(_lp(230, 2025, 6), _params(max_iter=4000, eps_abs=0.0, eps_rel=0.0)),
+           (_lp(2300, 9100, 8), _params(max_iter=1500, eps_abs=0.0, eps_rel=0.0)),
+           (_lp(40, 1700, 4), _params(max_iter=3000, eps_abs=0.0, eps_rel=0.0, precision="fp32"))]
+    lps = [lps[i] for i in order]
+
+    def run(group, budget):
+        with BatchEngine(max_slots=len(group)) as eng:
+            slots = [eng.admit(p, prm) for p, prm in group]
+            while eng.step(budget):
+                pass
+            return [(s.iterations, s.info.restarts, s.x.tobytes(), s.y.tobytes())
+                    for s in (eng.fetch(q) for q in slots)]
+
+    alone = [run([lp], 1 << 30)[0] for lp in lps]
+    assert run(lps, 1 << 30) == alone
+    assert run(lps, 700) == alone
+
+
+def test_more_lps_than_teams_take_turns():
+    """Beyond 256 LPs the team engine steps its LPs by one budget, so LPs on chip
+    stay there and take turns with it."""
+    small, large = _lp(63, 65, 5), _lp(2300, 9100, 8)
+    ps = _params(max_iter=500, eps_abs=0.0, eps_rel=0.0)
+    pl = _params(max_iter=300, eps_abs=0.0, eps_rel=0.0)
+    with BatchEngine(max_slots=270) as eng:
+        slots = [eng.admit(small, ps) for _ in range(266)] + [eng.admit(large, pl) for _ in range(3)]
+        while eng.step(400):
+            pass
+        got = [(s.iterations, s.x.tobytes(), s.y.tobytes()) for s in (eng.fetch(q) for q in slots)]
+    ref = [(b[0], b[7], b[8]) for b in (_bits([small], ps, True)[0], _bits([large], pl, True)[0])]
+    assert got == [ref[0]] * 266 + [ref[1]] * 3
