@@ -166,9 +166,10 @@ int pdlp_solve(const pdlp_problem_desc* prob, const pdlp_params* params,
                int32_t out_memory);
 
 /* ---- batched / served engine ------------------------------------------- *
- * A batch holds device-resident LPs ("slots") that one persistent kernel
- * advances together, each with its own step size, primal weight, restart
- * state and termination.  LPs may be admitted and retired between steps. */
+ * A batch holds device-resident LPs ("slots").  Those that fit the shared
+ * memory of a thread-block cluster are stepped there, one cluster each; one
+ * persistent kernel advances the others together.  Each has its own step
+ * size, primal weight, restart state and termination.  LPs may be admitted and retired between steps. */
 typedef struct pdlp_batch pdlp_batch;
 
 typedef struct pdlp_batch_config {
@@ -325,7 +326,8 @@ void pdlp_tune_cache_clear(void);
 
 /* y = A x, A in CSR with int64 pointers (backend.py:373-384).  Asynchronous
  * on `stream`; a fixed summation order, so repeated calls give the same bits.
- * Rows longer than 256 entries are summed by a second launch from a per-
+ * Rows longer than 256 entries are summed by a second launch (both launches
+ * are programmatic dependents of the one before) from a per-
  * (device, stream) list that the library keeps between calls.  It is
  * allocated on the first call with a given stream and grown when a larger m
  * comes; those calls synchronise the stream. */

@@ -1,4 +1,4 @@
-"""Batched engine: many LPs advanced together by one persistent kernel.
+"""Batched engine: many LPs advanced side by side on one GPU.
 
 ``BatchEngine`` wraps the ``pdlp_batch_*`` entry points of ``libpdlp_b200.so``.
 LPs are admitted into slots (their data is copied to the device and

@@ -7,8 +7,8 @@ device-resident LPs (``BatchEngine``) and runs a loop:
 2. admit queued requests while a slot is free and the LP fits the HBM
    budget -- the engine refuses an LP that does not fit
    (``PDLP_ERR_OOM``) and it waits in the queue until memory frees up;
-3. advance every admitted LP by a chunk of engine steps in one persistent
-   launch (their work overlaps on the device: one launch serves all of them);
+3. advance every admitted LP by a chunk of engine steps, side by side on the
+   device;
 4. fetch and retire the LPs that finished, recording the time from arrival to
    result.
 
