@@ -200,7 +200,10 @@ typedef struct pdlp_batch_config {
                                    without arriving, so the team's bounded
                                    wait runs out (a flag nothing sets); it
                                    exercises the timeout path without any
-                                   device fault                             */
+                                   device fault.  2: warps without work in a
+                                   pass read their team's state 20 us late
+                                   (results must not change).  Either keeps
+                                   every LP on block teams                  */
 } pdlp_batch_config;
 
 void pdlp_batch_config_default(pdlp_batch_config* cfg);

@@ -46,7 +46,7 @@ class BatchEngine:
         cfg.memory_budget = int(memory_budget)
         cfg.barrier_timeout_us = int(barrier_timeout_us)
         cfg.autotune = 1 if autotune else 0
-        cfg.test_withhold_arrival = 1 if test_withhold_arrival else 0
+        cfg.test_withhold_arrival = int(test_withhold_arrival)
         h = ctypes.c_void_p()
         code = self.lib.pdlp_batch_create(ctypes.byref(cfg), stream, ctypes.byref(h))
         if code == _lib.PDLP_ERR_CUDA:

@@ -82,6 +82,11 @@ __device__ int grid_barrier(Control* ctl, unsigned* counter, unsigned target,
   return flags[0];
 }
 
+// Test hook: about 20 us, longer than the passes of a small LP.
+__device__ void late_load() {
+  for (int i = 0; i < 20; ++i) __nanosleep(1000);
+}
+
 // One launch runs up to max_steps engine steps; every warp owns a fixed range
 // of row tiles and of column tiles for the whole launch.  The blocks form
 // teams that do not wait for one another: each team's tiles are the tiles of
@@ -92,7 +97,8 @@ __device__ int grid_barrier(Control* ctl, unsigned* counter, unsigned target,
 // every block of the team sees the same decision.
 //
 // A team of one LP (team_inst) keeps the LP's scheduling fields in its warps
-// (TeamCopy).  Its normal iterations then cost two barriers and nothing else:
+// (TeamCopy); they start from the State, which no pass may change before every
+// warp has read it, hence a barrier before the first step.  Its normal iterations then cost two barriers and nothing else:
 // no counters, no finisher, no state read.  Alone, in us per iteration with
 // checks and set-up: a 3 x 5 LP 16.2 -> 13.0, 230 x 2,025 20.4 -> 17.9.
 __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
@@ -123,11 +129,15 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
   const int inst = A.team_inst[team];              // the team's only LP, or -1
   State* const S = A.st + max(inst, 0);
   TeamCopy& C = W.team;
+  unsigned target = 0;
+  if (lane == 0) W.pass = 0;
   if (inst >= 0) {
     warp_inst(A, inst, W, lane);
+    if (A.late_loads && (r0 >= r1 || c0 >= c1)) late_load();
     team_load(C, S, lane);
+    target += nb;
+    if (!grid_barrier(A.ctl, bar, target, A.barrier_timeout_ns, nb == 1u, withhold, 1u)) return;
   }
-  unsigned target = 0;
 #ifdef PDLP_TRACE
   // phase timestamps of the first and the last block for the first steps
   long long* tr = nullptr;
@@ -166,8 +176,11 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
       if (!grid_barrier(A.ctl, bar, target, A.barrier_timeout_ns, nb == 1u, withhold, 1u)) return;
       if (lane == 0) fence_proxy_async_global();
       if (inst >= 0) {
-        if (C.rmode != R_ITER) team_load(C, S, lane);
-        else {
+        if (lane == 0) W.pass += 1;
+        if (C.rmode != R_ITER) {
+          if (A.late_loads && c0 >= c1) late_load();
+          team_read(A, W, lane);
+        } else {
           __syncwarp();
           if (lane == 0) C.ycommit = 0;              // this pass has retired it
           __syncwarp();
@@ -193,6 +206,7 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
                                 stop ? 1u + kStopBit : 1u);
     if (!go) return;
     if (lane == 0) fence_proxy_async_global();
+    if (inst >= 0 && lane == 0) W.pass += 1;
     if (quiet) {
       // the next state, as c_finish computes it for a normal step
       __syncwarp();
@@ -205,7 +219,8 @@ __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
       }
       __syncwarp();
     } else if (inst >= 0 && C.cmode != C_NONE) {
-      team_load(C, S, lane);
+      if (A.late_loads && (r0 >= r1 || c0 >= c1)) late_load();
+      team_read(A, W, lane);
     }
     PDLP_STAMP(step, 4);
     if (go & 2) { ++step; break; }
@@ -481,6 +496,9 @@ thread_local std::string g_err;
 
 constexpr size_t kAlign = 256;
 
+// pdlp_batch_config.test_withhold_arrival
+constexpr int kTestWithhold = 1, kTestLateLoads = 2;
+
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 int default_tile_rows() { return kWTileRows; }
@@ -572,6 +590,7 @@ struct pdlp_batch {
   Inst* d_inst = nullptr;
   State* d_state = nullptr;
   unsigned* d_counters = nullptr;
+  TeamCopy* d_team_copies = nullptr;   // two per slot (TeamCopy)
   Control* d_ctl = nullptr;
   Tile* d_rtiles = nullptr;
   Tile* d_ctiles = nullptr;
@@ -950,6 +969,8 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
   }
   *count = (int)order.size();
   if (order.empty()) return PDLP_OK;
+  EngineArgs R = A;
+  R.team_copies = nullptr;           // the clusters' warps read the State (engine_resident)
   cudaStream_t st = b->stream;
   PDLP_CUDA(cudaMemcpyAsync(b->d_res, b->h_res, sizeof(ResidentLP) * order.size(), cudaMemcpyHostToDevice, st));
   // one size: on the batch's stream; several: side by side on streams of
@@ -976,7 +997,7 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
       cudaLaunchConfig_t cfg;
       cudaLaunchAttribute attr;
       res_config(1 << k, (int)(z - a), q, &cfg, &attr);
-      PDLP_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel(f32 != 0), A,
+      PDLP_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel(f32 != 0), R,
                                    (const ResidentLP*)(b->d_res + first + a),
                                    b->d_res_steps + first + a));
       count_launches(1);
@@ -1937,6 +1958,7 @@ int pdlp_batch_create(const pdlp_batch_config* cfg, void* stream, pdlp_batch** o
   if ((e = cudaMalloc(&b->d_inst, sizeof(Inst) * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = cudaMalloc(&b->d_state, sizeof(State) * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = cudaMalloc(&b->d_counters, sizeof(unsigned) * 2 * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
+  if ((e = cudaMalloc(&b->d_team_copies, sizeof(TeamCopy) * 2 * c.max_slots)) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = cudaMalloc(&b->d_ctl, sizeof(Control))) != cudaSuccess) return bail(e, "cudaMalloc");
   if ((e = cudaMallocHost(&b->h_ctl, sizeof(Control))) != cudaSuccess) return bail(e, "cudaMallocHost");
   if ((e = cudaMalloc(&b->d_raypart, sizeof(double) * 16 * kRayBlocks)) != cudaSuccess)
@@ -1968,6 +1990,7 @@ int pdlp_batch_destroy(pdlp_batch* b) {
   for (auto& s : b->slots) if (s.arena) cudaFree(s.arena);
   for (auto& a : b->spare) cudaFree(a.first);
   cudaFree(b->d_inst); cudaFree(b->d_state); cudaFree(b->d_counters); cudaFree(b->d_ctl);
+  cudaFree(b->d_team_copies);
   cudaFree(b->d_rtiles); cudaFree(b->d_ctiles); cudaFree(b->d_rwarp); cudaFree(b->d_cwarp);
   cudaFree(b->d_teams);
   cudaFree(b->d_partials); cudaFree(b->d_group_tiles); cudaFree(b->d_gpartials);
@@ -2038,6 +2061,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
 #endif
   A.inst = b->d_inst; A.st = b->d_state;
   A.counters = b->d_counters; A.ctl = b->d_ctl;
+  A.team_copies = b->cfg.persistent ? b->d_team_copies : nullptr;
   A.barrier_timeout_ns = b->cfg.barrier_timeout_us > 0 ? b->cfg.barrier_timeout_us * 1000LL
                                                        : 4000000000LL;
   A.n_inst = (int)b->slots.size();
@@ -2069,7 +2093,9 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     A.partials = b->d_partials; A.gpartials = b->d_gpartials; A.gcounters = b->d_gcounters;
     const int64_t chunk = std::min(most, kChunk);
     A.max_steps = b->cfg.persistent ? kChunk : chunk;
-    A.withhold_block = (b->cfg.persistent && b->cfg.test_withhold_arrival) ? b->withhold_candidate : -1;
+    A.withhold_block = (b->cfg.persistent && b->cfg.test_withhold_arrival == kTestWithhold)
+                           ? b->withhold_candidate : -1;
+    A.late_loads = b->cfg.test_withhold_arrival == kTestLateLoads;
     b->h_ctl->bar_count = 0; b->h_ctl->bar_gen = 0; b->h_ctl->active = b->n_running;
     b->h_ctl->error = 0; b->h_ctl->error_where = 0; b->h_ctl->stop = 0; b->h_ctl->idle = 0;
     b->h_ctl->team_active[kMaxTeams] = (int)b->resident.size();

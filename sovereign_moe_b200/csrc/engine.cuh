@@ -175,6 +175,8 @@ struct Control {
   int team_steps[kMaxTeams];          // steps each team completed (its leader, at exit)
 };
 
+struct TeamCopy;          // engine_device.cuh
+
 struct EngineArgs {
   Inst* inst;
   State* st;
@@ -186,6 +188,8 @@ struct EngineArgs {
   const int* team_blocks;   // [n_teams] blocks per team
   const int* team_first;    // [n_teams] first block of each team (its leader)
   const int* team_inst;     // [n_teams] the team's only instance, -1 for a team of several
+  TeamCopy* team_copies;    // [2 * n_inst] what a finisher tells its team (team_publish);
+                            // null where no warp reads it
   const int2* group_tiles;  // [n_groups]: tile range of each group (row groups first)
   int n_rgroups, n_groups;
   double* partials;         // [(n_rtiles + n_ctiles) * kNP] tile partials
@@ -197,6 +201,7 @@ struct EngineArgs {
   long long barrier_timeout_ns;
   int withhold_block;       // test hook: this block leaves at its first barrier
                             // without arriving (-1: none)
+  int late_loads;           // test hook: warps without tiles read their copies late
   int n_inst;
   long long* trace;         // tracing builds only: phase timestamps, else null
 };

@@ -29,7 +29,16 @@ constexpr unsigned kFull = 0xffffffffu;
 // copy by itself: no counters, no finisher, no state writes and no reload.
 // `pend` counts the iterations the copy is ahead of the State in memory; the
 // next finisher, or the team's leader at the end of the launch, writes them
-// down first.  After every other pass the warps reload the copy.
+// down first.
+//
+// After every other pass the warps take the copy anew, from what the pass's
+// finisher published (team_publish), never from the State: a warp that owns no
+// tile of the next pass does not hold up that pass's finisher, so the State may
+// change while it reads.  Each LP has two published copies, used in turn by
+// the passes its team has run in the launch: the finisher of pass p writes
+// copy (p + 1) mod 2, which the warps read after the barrier that ends p.  The
+// next to write that copy is the finisher of pass p + 2 at the earliest, after
+// the barrier that ends p + 1, which every warp meets once it has read.
 struct TeamCopy {
   double eta, omega;
   long long k;
@@ -52,7 +61,8 @@ struct __align__(16) WarpSmem {
   double s1[kWTileRows];               // row sums, second right-hand side
   TeamCopy team;
   int inst_id;
-  int pad[3];
+  unsigned pass;                       // passes the team has run in this launch
+  int pad[2];
   Inst inst;                           // cached descriptor of inst_id
 };
 static_assert(sizeof(TeamCopy) % 16 == 0, "WarpSmem layout");

@@ -87,6 +87,44 @@ __device__ __forceinline__ void team_load(TeamCopy& c, const State* S, int lane)
   __syncwarp();
 }
 
+// The copy as the finisher of the team's last pass published it.
+__device__ __forceinline__ void team_read(const EngineArgs& A, WarpSmem& W, int lane) {
+  __syncwarp();
+  if (lane == 0) {
+    const TeamCopy* p = A.team_copies + 2 * (size_t)W.inst_id + (W.pass & 1u);
+    TeamCopy& c = W.team;
+    const double eta = ld_mut(&p->eta), omega = ld_mut(&p->omega);
+    const long long k = ld_mut(&p->k);
+    const int rmode = ld_mut(&p->rmode), cmode = ld_mut(&p->cmode), cprimal = ld_mut(&p->cprimal);
+    const int xcommit = ld_mut(&p->xcommit), ycommit = ld_mut(&p->ycommit);
+    c.eta = eta;
+    c.omega = omega;
+    c.k = k;
+    c.rmode = rmode;
+    c.cmode = cmode;
+    c.cprimal = cprimal;
+    c.xcommit = xcommit;
+    c.ycommit = ycommit;
+    c.pend = 0;
+  }
+  __syncwarp();
+}
+
+// By the finishing thread of a pass, once it has advanced the state: the fields
+// the team's warps read after the barrier that ends the pass (TeamCopy).
+__device__ __forceinline__ void team_publish(const EngineArgs& A, const WarpSmem& W, const State* S) {
+  if (A.team_copies == nullptr) return;
+  TeamCopy* o = A.team_copies + 2 * (size_t)W.inst_id + ((W.pass + 1u) & 1u);
+  o->eta = S->eta;
+  o->omega = S->omega;
+  o->k = S->k;
+  o->rmode = S->rmode;
+  o->cmode = S->cmode;
+  o->cprimal = S->cprimal;
+  o->xcommit = S->xcommit;
+  o->ycommit = S->ycommit;
+}
+
 // Writes down what the copy is ahead of the state: its normal iterations, one
 // addition to sum_eta each, as c_finish makes them, and the modes they lead
 // to.  By one thread, when every tile of those iterations has completed.
@@ -509,6 +547,7 @@ __device__ void hot_rtile(const EngineArgs& A, const Tile& t, int ti, const Inst
     if (lane == 0) {
       if (team) team_flush(*team, S);
       r_finish(A, I, S, rmode, res);
+      if (team) team_publish(A, W, S);
     }
     __syncwarp();
   }
@@ -593,6 +632,7 @@ __device__ void hot_ctile(const EngineArgs& A, const Tile& t, int ti, const Inst
     if (lane == 0) {
       if (team) team_flush(*team, S);
       c_finish(A, I, S, cmode, res);
+      if (team) team_publish(A, W, S);
     }
     __syncwarp();
   }
@@ -902,6 +942,7 @@ __device__ void process_rtile(const EngineArgs& A, const Tile t, int ti, WarpSme
     if (lane == 0) {
       if (team) team_flush(*team, S);
       r_finish(A, I, S, rmode, res);
+      if (team) team_publish(A, W, S);
     }
     __syncwarp();
   }
@@ -1418,6 +1459,7 @@ __device__ void process_ctile(const EngineArgs& A, const Tile t, int ti, WarpSme
     if (lane == 0) {
       if (team) team_flush(*team, S);
       c_finish(A, I, S, cmode, res);
+      if (team) team_publish(A, W, S);
     }
     __syncwarp();
   }

@@ -725,6 +725,12 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
   int turn = 0;
   bool started = false;                // every CTA has met a barrier of this kernel
   while (step < lp.budget) {
+    // A warp without tiles in a pass may still be reading the State while that
+    // pass's finisher writes it.  It takes the same way through the barriers
+    // all the same: before an A pass of this loop rmode alone decides, and no A
+    // pass's finisher changes it (a line search runs in res_run); a step
+    // without an A pass is a C_PRIMAL, in res_run, which copies the State
+    // before a barrier; and the second load below decides no barrier.
     team_load(C, S, lane);
     if (C.rmode == R_NONE && C.cmode == C_NONE) break;           // the LP is done
     if (res_hot(C.rmode, C.cmode)) {
