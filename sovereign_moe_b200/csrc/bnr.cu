@@ -80,8 +80,7 @@ template <int V>
 __global__ void __launch_bounds__(256, 8) bnr_spmm(int rows, int k, const int64_t* __restrict__ rp,
                                                 const int* __restrict__ ri,
                                                 const double* __restrict__ rx,
-                                                const double* __restrict__ X,
-                                                double* __restrict__ Y) {
+                                                const double* X, double* Y) {
   constexpr int kBatch = 2;
   grid_dep_wait();
   const int groups = k / V;
@@ -201,7 +200,7 @@ template <int V>
 __device__ __forceinline__ Lanes<V> bnr_row(const BnrStage& S, bool staged, int r, int k,
                                             const int* __restrict__ ri,
                                             const double* __restrict__ rx,
-                                            const double* __restrict__ Xc) {
+                                            const double* Xc) {
   constexpr int kB = 4;
   Lanes<V> a;
 #pragma unroll
@@ -240,7 +239,7 @@ __device__ __forceinline__ Lanes<V> bnr_row(const BnrStage& S, bool staged, int 
 // The block's sums per node from the rows' terms; NS sums.
 template <int V, int NS>
 __device__ __forceinline__ void bnr_sums(BnrStage& S, const BnrTile<V>& t, int k, int pstride,
-                                         int part_block, double* __restrict__ part) {
+                                         int part_block, double* part) {
   const int tile = t.tile;
   __syncthreads();                    // the rows' terms are in place
   for (int w = threadIdx.x; w < 8 * tile; w += kBnrThreads) {
@@ -287,10 +286,9 @@ template <int V>
 __global__ void __launch_bounds__(kBnrThreads, 2) bnr_cols(
     int n, int k, int txs, int mblocks, int pstride, const int64_t* __restrict__ cp,
     const int* __restrict__ ci, const double* __restrict__ cx, const double* __restrict__ c,
-    const double* __restrict__ eta, const double* __restrict__ eta_prev,
-    const double* __restrict__ omega, const int* __restrict__ pend, double* __restrict__ X,
-    double* __restrict__ AtY, const double* __restrict__ dY, const double* __restrict__ L,
-    const double* __restrict__ U, double* __restrict__ dX, double* __restrict__ part) {
+    const double* eta, const double* eta_prev, const double* __restrict__ omega, const int* pend,
+    double* X, double* AtY, const double* dY, const double* __restrict__ L,
+    const double* __restrict__ U, double* dX, double* part) {
   __shared__ BnrStage S;
   const BnrTile<V> t = bnr_tile<V>(n, k, txs);
   const int r0 = blockIdx.x * kRowsPerBlock;
@@ -352,10 +350,9 @@ template <int V>
 __global__ void __launch_bounds__(kBnrThreads, 2) bnr_rows(
     int m, int k, int txs, int pstride, const int64_t* __restrict__ rp, const int* __restrict__ ri,
     const double* __restrict__ rx, const double* __restrict__ rl, const double* __restrict__ ru,
-    const double* __restrict__ eta, const double* __restrict__ eta_prev,
-    const double* __restrict__ omega, const int* __restrict__ pend, double* __restrict__ Y,
-    double* __restrict__ AX, const double* __restrict__ AdX_prev, const double* __restrict__ dX,
-    double* __restrict__ AdX, double* __restrict__ dY, double* __restrict__ part) {
+    const double* eta, const double* eta_prev, const double* __restrict__ omega, const int* pend,
+    double* Y, double* AX, const double* AdX_prev, const double* dX, double* AdX, double* dY,
+    double* part) {
   __shared__ BnrStage S;
   const BnrTile<V> t = bnr_tile<V>(m, k, txs);
   const int r0 = blockIdx.x * kRowsPerBlock;
@@ -410,7 +407,7 @@ __global__ void __launch_bounds__(kBnrThreads, 2) bnr_rows(
 // with threadIdx.x the node within a 32-node tile; same sums, same order.
 __device__ __forceinline__ void bnr_block_sums(double s0, double s1, int k, int node,
                                                int pstride, int part_block,
-                                               double* __restrict__ part) {
+                                               double* part) {
   __shared__ double sh[2][8][32];
   sh[0][threadIdx.y][threadIdx.x] = s0;
   sh[1][threadIdx.y][threadIdx.x] = s1;
@@ -431,17 +428,13 @@ __device__ __forceinline__ void bnr_block_sums(double s0, double s1, int k, int 
 // node's sum of dX dX over the block's rows.
 __global__ void __launch_bounds__(256) bnr_primal(int n, int k, int mblocks, int pstride,
                                                   const double* __restrict__ c,
-                                                  const double* __restrict__ eta,
-                                                  const double* __restrict__ eta_prev,
+                                                  const double* eta, const double* eta_prev,
                                                   const double* __restrict__ omega,
-                                                  const int* __restrict__ pend,
-                                                  double* __restrict__ X,
-                                                  double* __restrict__ AtY,
-                                                  const double* __restrict__ AtdY,
+                                                  const int* pend, double* X, double* AtY,
+                                                  const double* AtdY,
                                                   const double* __restrict__ L,
                                                   const double* __restrict__ U,
-                                                  double* __restrict__ dX,
-                                                  double* __restrict__ part) {
+                                                  double* dX, double* part) {
   grid_dep_wait();
   const int node = blockIdx.y * 32 + threadIdx.x;
   double s = 0.0;
@@ -475,15 +468,11 @@ __global__ void __launch_bounds__(256) bnr_primal(int n, int k, int mblocks, int
 __global__ void __launch_bounds__(256) bnr_dual(int m, int k, int pstride,
                                                 const double* __restrict__ rl,
                                                 const double* __restrict__ ru,
-                                                const double* __restrict__ eta,
-                                                const double* __restrict__ eta_prev,
+                                                const double* eta, const double* eta_prev,
                                                 const double* __restrict__ omega,
-                                                const int* __restrict__ pend,
-                                                double* __restrict__ Y, double* __restrict__ AX,
-                                                const double* __restrict__ AdX_prev,
-                                                const double* __restrict__ AdX,
-                                                double* __restrict__ dY,
-                                                double* __restrict__ part) {
+                                                const int* pend, double* Y, double* AX,
+                                                const double* AdX_prev, const double* AdX,
+                                                double* dY, double* part) {
   grid_dep_wait();
   const int node = blockIdx.y * 32 + threadIdx.x;
   double s0 = 0.0, s1 = 0.0;
@@ -536,11 +525,9 @@ __device__ __forceinline__ double warp_blocks_sum(const double* __restrict__ par
 // 1 + t^-damp), computed on the host with the C library's pow, as the
 // reference computes them.
 __global__ void __launch_bounds__(128) bnr_accept(int k, int mblocks, int nblocks,
-                                                  const double* __restrict__ part,
-                                                  double* __restrict__ eta,
-                                                  double* __restrict__ eta_prev,
-                                                  const double* __restrict__ omega,
-                                                  int* __restrict__ accept,
+                                                  const double* part, double* eta,
+                                                  double* eta_prev,
+                                                  const double* __restrict__ omega, int* accept,
                                                   const double* __restrict__ fac) {
   const int lane = threadIdx.x & 31;
   const int node = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

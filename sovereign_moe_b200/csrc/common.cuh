@@ -70,6 +70,13 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 // once when there is none); grid_dep_release lets the next kernel in the
 // stream, if it was launched as a programmatic dependent, start its CTAs as
 // this kernel's CTAs leave the SMs.
+//
+// A kernel launched as a programmatic dependent may begin while launches before
+// it still write what it reads.  It reads such arrays after grid_dep_wait, as
+// ordinary loads through plain pointers: a `const __restrict__` pointer or __ldg
+// says that nobody writes the array while the kernel lives, which lets the
+// compiler use the read-only path and place the load before the wait; even a
+// written `__restrict__` pointer says that the wait cannot change its data.
 __device__ __forceinline__ void grid_dep_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -68,9 +68,7 @@ constexpr int kBandCap = 3072;         // x entries a block stages (banded varia
 template <typename T>
 __device__ __forceinline__ void spmv_rows_staged(int r0, int i0, int i1, long long rs,
                                                  long long re, long long p0, int cnt, int lane,
-                                                 const int* __restrict__ ri,
-                                                 const T* __restrict__ rx,
-                                                 const T* __restrict__ x, T* __restrict__ y,
+                                                 const int* ri, const T* rx, const T* x, T* y,
                                                  T* __restrict__ prod,
                                                  const T* band = nullptr, int blo = 0,
                                                  int bcnt = 0) {
@@ -80,15 +78,15 @@ __device__ __forceinline__ void spmv_rows_staged(int r0, int i0, int i1, long lo
 #pragma unroll
     for (int u = 0; u < kStageUnroll; ++u) {
       const int q = q0 + u * 32 + lane;
-      idx[u] = q < cnt ? __ldg(ri + p0 + q) : 0;
-      val[u] = q < cnt ? __ldg(rx + p0 + q) : T(0);
+      idx[u] = q < cnt ? ri[p0 + q] : 0;
+      val[u] = q < cnt ? rx[p0 + q] : T(0);
     }
     T xv[kStageUnroll];
 #pragma unroll
     for (int u = 0; u < kStageUnroll; ++u) {
       const int q = q0 + u * 32 + lane;
       const unsigned off = (unsigned)(idx[u] - blo);
-      xv[u] = q < cnt ? (off < (unsigned)bcnt ? band[off] : __ldg(x + idx[u])) : T(0);
+      xv[u] = q < cnt ? (off < (unsigned)bcnt ? band[off] : x[idx[u]]) : T(0);
     }
 #pragma unroll
     for (int u = 0; u < kStageUnroll; ++u) {
@@ -133,9 +131,7 @@ __device__ __forceinline__ int spmv_next_run(int start, int nr, long long rs, lo
 template <typename T, int L>
 __device__ __forceinline__ void spmv_block_rows(int r0, int nr, long long rs, long long re,
                                                 unsigned long_mask, int lane,
-                                                const int* __restrict__ ri,
-                                                const T* __restrict__ rx,
-                                                const T* __restrict__ x, T* __restrict__ y) {
+                                                const int* ri, const T* rx, const T* x, T* y) {
   constexpr int G = 32 / L;
   const int sub = lane & (L - 1), gi = lane / L;
   for (int g = 0; g < nr; g += G) {
@@ -146,7 +142,7 @@ __device__ __forceinline__ void spmv_block_rows(int r0, int nr, long long rs, lo
     T acc = T(0);
     if (active) {
 #pragma unroll 4
-      for (long long p = p0 + sub; p < p1; p += L) acc += __ldg(rx + p) * __ldg(x + __ldg(ri + p));
+      for (long long p = p0 + sub; p < p1; p += L) acc += rx[p] * x[ri[p]];
     }
 #pragma unroll
     for (int off = L >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(kAll, acc, off);
@@ -156,9 +152,8 @@ __device__ __forceinline__ void spmv_block_rows(int r0, int nr, long long rs, lo
 
 template <typename T>
 __global__ void __launch_bounds__(kSpmvWarps * 32, sizeof(T) == 8 ? 6 : 0) spmv_rows_kernel(
-    int m, const int64_t* __restrict__ rp, const int* __restrict__ ri,
-    const T* __restrict__ rx, const T* __restrict__ x, T* __restrict__ y,
-    int* __restrict__ long_rows, int rows_per_warp) {
+    int m, const int64_t* rp, const int* ri, const T* rx, const T* x, T* y, int* long_rows,
+    int rows_per_warp) {
   __shared__ T stage[kSpmvWarps][kStageEntries];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // both launches of a call are programmatic dependents of the launch before
@@ -171,8 +166,8 @@ __global__ void __launch_bounds__(kSpmvWarps * 32, sizeof(T) == 8 ? 6 : 0) spmv_
   if (b * rows_per_warp >= m) return;               // whole warps leave together
   const int r0 = (int)(b * rows_per_warp);
   const int nr = min(rows_per_warp, m - r0);
-  const long long rs = lane < nr ? (long long)__ldg(rp + r0 + lane) : 0LL;
-  const long long re = lane < nr ? (long long)__ldg(rp + r0 + lane + 1) : 0LL;
+  const long long rs = lane < nr ? (long long)rp[r0 + lane] : 0LL;
+  const long long re = lane < nr ? (long long)rp[r0 + lane + 1] : 0LL;
   const bool is_long = lane < nr && re - rs > kLongRow;
   if (is_long) {
     // a count left over by a failed earlier call cannot push a write past
@@ -194,17 +189,15 @@ __global__ void __launch_bounds__(kSpmvWarps * 32, sizeof(T) == 8 ? 6 : 0) spmv_
 
 template <typename T>
 __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_groups_kernel(
-    int m, const int64_t* __restrict__ rp, const int* __restrict__ ri,
-    const T* __restrict__ rx, const T* __restrict__ x, T* __restrict__ y,
-    int* __restrict__ long_rows) {
+    int m, const int64_t* rp, const int* ri, const T* rx, const T* x, T* y, int* long_rows) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   grid_dep_wait();
   const long long b = (long long)blockIdx.x * kSpmvWarps + w;
   if (b * 32 >= m) return;                          // whole warps leave together
   const int r0 = (int)(b * 32);
   const int nr = min(32, m - r0);
-  const long long rs = lane < nr ? (long long)__ldg(rp + r0 + lane) : 0LL;
-  const long long re = lane < nr ? (long long)__ldg(rp + r0 + lane + 1) : 0LL;
+  const long long rs = lane < nr ? (long long)rp[r0 + lane] : 0LL;
+  const long long re = lane < nr ? (long long)rp[r0 + lane + 1] : 0LL;
   const bool is_long = lane < nr && re - rs > kLongRow;
   if (is_long) {
     const int slot = atomicAdd(long_rows, 1);
@@ -236,9 +229,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_groups_kernel(
 // variants.
 template <typename T>
 __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_band_kernel(
-    int m, const int64_t* __restrict__ rp, const int* __restrict__ ri,
-    const T* __restrict__ rx, const T* __restrict__ x, T* __restrict__ y,
-    int* __restrict__ long_rows) {
+    int m, const int64_t* rp, const int* ri, const T* rx, const T* x, T* y, int* long_rows) {
   __shared__ T stage[kSpmvWarps][kStageEntries];
   __shared__ T band[kBandCap];
   __shared__ int wlo[kSpmvWarps], whi[kSpmvWarps];
@@ -249,8 +240,8 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_band_kernel(
   const bool have = b < nblk;                       // warp-uniform
   const int r0 = have ? (int)(b * 32) : 0;
   const int nr = have ? min(32, m - r0) : 0;
-  const long long rs = lane < nr ? (long long)__ldg(rp + r0 + lane) : 0LL;
-  const long long re = lane < nr ? (long long)__ldg(rp + r0 + lane + 1) : 0LL;
+  const long long rs = lane < nr ? (long long)rp[r0 + lane] : 0LL;
+  const long long re = lane < nr ? (long long)rp[r0 + lane + 1] : 0LL;
   const bool is_long = lane < nr && re - rs > kLongRow;
   if (is_long) {
     const int slot = atomicAdd(long_rows, 1);
@@ -265,7 +256,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_band_kernel(
     const int end = spmv_next_run(start, nr, rs, re, long_mask, lane);
     const long long qa = __shfl_sync(kAll, rs, start), qb = __shfl_sync(kAll, re, end - 1);
     for (long long q = qa + lane; q < qb; q += 32) {
-      const int j = __ldg(ri + q);
+      const int j = ri[q];
       lo = min(lo, j);
       hi = max(hi, j);
     }
@@ -281,7 +272,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_band_kernel(
   int blo = 0x7fffffff, bhi = -1;
   for (int k = 0; k < kSpmvWarps; ++k) { blo = min(blo, wlo[k]); bhi = max(bhi, whi[k]); }
   const int bcnt = (bhi >= blo && bhi - blo < kBandCap) ? bhi - blo + 1 : 0;   // block-uniform
-  for (int i = threadIdx.x; i < bcnt; i += kSpmvWarps * 32) band[i] = __ldg(x + blo + i);
+  for (int i = threadIdx.x; i < bcnt; i += kSpmvWarps * 32) band[i] = x[blo + i];
   __syncthreads();
   for (int start = 0; start < nr;) {
     if ((long_mask >> start) & 1u) { ++start; continue; }
@@ -295,8 +286,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_band_kernel(
 
 template <typename T>
 __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_long_rows_kernel(
-    const int64_t* __restrict__ rp, const int* __restrict__ ri, const T* __restrict__ rx,
-    const T* __restrict__ x, T* __restrict__ y, int m, int* __restrict__ long_rows) {
+    const int64_t* rp, const int* ri, const T* rx, const T* x, T* y, int m, int* long_rows) {
   __shared__ T part[kSpmvWarps];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -306,7 +296,7 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_long_rows_kernel(
   for (int k = blockIdx.x; k < count; k += gridDim.x) {
     const int r = long_rows[2 + k];
     if (r < 0 || r >= m) continue;    // only after a failed earlier call (block-uniform)
-    const long long p0 = __ldg(rp + r), p1 = __ldg(rp + r + 1);
+    const long long p0 = rp[r], p1 = rp[r + 1];
     T sum = T(0);
     for (long long base = p0 + 128LL * w; base < p1; base += 128LL * kSpmvWarps) {
       int idx[4];
@@ -314,13 +304,13 @@ __global__ void __launch_bounds__(kSpmvWarps * 32) spmv_long_rows_kernel(
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const long long p = base + lane + 32 * u;
-        idx[u] = p < p1 ? __ldg(ri + p) : 0;
-        val[u] = p < p1 ? __ldg(rx + p) : T(0);
+        idx[u] = p < p1 ? ri[p] : 0;
+        val[u] = p < p1 ? rx[p] : T(0);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const long long p = base + lane + 32 * u;
-        if (p < p1) sum += val[u] * __ldg(x + idx[u]);
+        if (p < p1) sum += val[u] * x[idx[u]];
       }
     }
 #pragma unroll

@@ -221,7 +221,7 @@ __device__ __forceinline__ PlanTile shfl_tile(const PlanTile& mine, int j) {
 // gathers read shared memory only.
 template <typename T, bool STAGED>
 __device__ __forceinline__ void consume_tile(const PlanTile& t, const unsigned char* st,
-                                             const T* __restrict__ x, T* __restrict__ y,
+                                             const T* x, T* y,
                                              const int* __restrict__ long_rows, long long base,
                                              int gw, int lane) {
   using L = StageLayout<T>;
@@ -234,7 +234,7 @@ __device__ __forceinline__ void consume_tile(const PlanTile& t, const unsigned c
   // a rewritten index: staged x (window or halo), or -(column + 1)
   auto xval = [&](int jj) -> T {
     if (STAGED) return sx[jj];
-    return jj >= 0 ? sx[jj] : __ldg(x + (-1 - jj));
+    return jj >= 0 ? sx[jj] : x[-1 - jj];
   };
   // the short rows, one per lane, in the plan's order: the 32 rows of a warp
   // start at different banks, so the lanes' loads of indices and values do
@@ -299,8 +299,8 @@ template <typename T>
 __global__ void __launch_bounds__(kPlanThreads, 1) spmv_plan_kernel(
 
     const PlanTile* __restrict__ tiles, const int* __restrict__ cta_first,
-    const int64_t* __restrict__ rp, const int* __restrict__ idx, const T* __restrict__ rx,
-    const T* __restrict__ x, T* __restrict__ y, const int* __restrict__ long_rows,
+    const int64_t* __restrict__ rp, const int* __restrict__ idx, const T* rx, const T* x, T* y,
+    const int* __restrict__ long_rows,
     const int* __restrict__ halo_cols, const uint16_t* __restrict__ perm, long long base,
     int* status) {
   using L = StageLayout<T>;
@@ -432,10 +432,10 @@ __global__ void __launch_bounds__(kPlanThreads, 1) spmv_plan_kernel(
       __syncwarp();
       if (c0 == 0) grid_dep_wait();          // x is the caller's
       int col = hcols[0][lane];
-      T cur = col >= 0 ? __ldg(x + col) : T(0);
+      T cur = col >= 0 ? x[col] : T(0);
       for (int j = 0; j < cn; ++j, ++k) {
         const int nc = j + 1 < cn ? hcols[j + 1][lane] : -1;
-        const T nxt = nc >= 0 ? __ldg(x + nc) : T(0);
+        const T nxt = nc >= 0 ? x[nc] : T(0);
         const int s = k % kPlanStages;
         int go = 1;
         if (lane == 0) {
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) spmv_plan_kernel(
         T a = T(0);
         const long long end = t.p0 + t.cnt;
         for (long long q = t.p0 + lane; q < end; q += 32)
-          a = add_rn(a, mul_rn(__ldg(rx + base + q), __ldg(x + (-1 - __ldg(idx + q)))));
+          a = add_rn(a, mul_rn(rx[base + q], x[-1 - __ldg(idx + q)]));
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) a = add_rn(a, __shfl_xor_sync(kAllLanes, a, off));
         if (lane == 0) y[t.r0] = a;
