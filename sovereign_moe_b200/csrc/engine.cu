@@ -2435,6 +2435,24 @@ int pdlp_batch_cancel(pdlp_batch* b, int32_t slot) {
   return PDLP_OK;
 }
 
+#ifdef PDLP_BOUNDS_CHECK
+// Bounds-checked builds, for their tests: overwrites one entry of an admitted
+// slot's row indices (which = 0), column indices (1), row pointers (2) or
+// column pointers (3), which admission has checked.
+int pdlp_batch_test_overwrite(pdlp_batch* b, int32_t slot, int32_t which, int64_t at, int32_t value) {
+  if (!b || slot < 0 || slot >= (int)b->slots.size() || !b->slots[slot].used)
+    return fail(PDLP_ERR_ARG, "no such slot");
+  const Inst& I = b->slots[slot].inst;
+  const int* const arrays[4] = {I.ri, I.ci, I.rp, I.cp};
+  const int64_t len[4] = {I.nnz, I.nnz, (int64_t)I.m + 1, (int64_t)I.n + 1};
+  if (which < 0 || which > 3 || at < 0 || at >= len[which]) return fail(PDLP_ERR_ARG, "out of range");
+  PDLP_CUDA(cudaMemcpyAsync(const_cast<int*>(arrays[which]) + at, &value, sizeof(int),
+                            cudaMemcpyHostToDevice, b->stream));
+  PDLP_CUDA(cudaStreamSynchronize(b->stream));
+  return PDLP_OK;
+}
+#endif
+
 void pdlp_tune_key_of(int32_t m, int32_t n, int64_t nnz, pdlp_tune_key* key) {
   if (key) *key = tune_key(m, n, nnz);
 }

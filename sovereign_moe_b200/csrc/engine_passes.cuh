@@ -340,9 +340,12 @@ __device__ void c_finish(const EngineArgs& A, const Inst& I, State* S, int cmode
 // generic passes' (same operands, same order).
 
 // Bounds-checked builds (-DPDLP_BOUNDS_CHECK) test every gathered index
-// against the source vector's length and every staged row pointer against the
-// tile: a failure records PDLP_ERR_BOUNDS (the launch ends at its next grid
-// barrier) and the access is skipped.  Product builds compile none of it.
+// of a normal tile's iteration, line search or primal step against the source
+// vector's length, and every staged row pointer against the tile; for LPs on
+// chip when the share of a cluster's CTA is loaded (engine_resident.cuh).  A
+// failure records PDLP_ERR_BOUNDS (the launch ends at its next grid barrier, a
+// cluster before it steps) and the access is skipped.  Product builds compile
+// none of it.
 #ifdef PDLP_BOUNDS_CHECK
 __device__ __forceinline__ bool index_ok(const EngineArgs& A, int i, int n, int where) {
   if ((unsigned)i < (unsigned)n) return true;

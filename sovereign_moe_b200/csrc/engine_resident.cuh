@@ -49,7 +49,8 @@ constexpr int kResMaxCluster = 16;
 struct __align__(16) ResHeader {
   int flags[4];            // block_flags()
   int failed[2];           // rank 0's view of the launch's error word, by generic step
-  int pad[2];
+  int bad;                 // bounds-checked builds: a check of some CTA's resident data failed
+  int pad;
   Inst inst;
   State st;
   TeamCopy team[kResWarps];
@@ -400,9 +401,33 @@ __device__ __forceinline__ bool res_hot(int rmode, int cmode) {
 
 // ---- a run of iterations --------------------------------------------------------
 
+// Row pointer i of a CTA's share (`rows` rows, cnt entries from entry base on).
+// Bounds-checked builds test it as tile_ptrs_ok does and keep it in the share.
+__device__ __forceinline__ int res_pointer(const EngineArgs& A, const int* ptr, int i, int rows,
+                                           int base, int cnt, int where) {
+  if (rows == 0) return 0;
+  const int v = ld_ro(ptr + i) - base;
+#ifdef PDLP_BOUNDS_CHECK
+  const int next = i < rows ? ld_ro(ptr + i + 1) - base : cnt;
+  if (v < 0 || v > next || next > cnt || (i == 0 && v != 0) || (i == rows && v != cnt)) {
+    if (atomicCAS(&A.ctl->error, 0, PDLP_ERR_BOUNDS) == 0) A.ctl->error_where = where;
+    block_fail();
+    return min(max(v, 0), cnt);
+  }
+#endif
+  return v;
+}
+
+// Index j of an entry, below len: index_ok's test before the index is narrowed;
+// a bad one is kept out of the products.
+__device__ __forceinline__ uint16_t res_index(const EngineArgs& A, int j, int len, int where) {
+  return index_ok(A, j, len, where) ? (uint16_t)j : (uint16_t)0;
+}
+
 // Steps the LP from global memory's state until a mode that does not run on
 // chip, or until `step` reaches the budget.  Returns the step count; the
-// vectors and the state are back in global memory then.
+// vectors and the state are back in global memory then.  (-1, with nothing
+// stepped: bounds-checked builds, when a check of the loaded data failed.)
 template <typename T>
 __device__ __forceinline__ int res_run(const EngineArgs& A, const ResidentLP& lp, State* S, int rank,
                                        int size, int step) {
@@ -455,15 +480,15 @@ __device__ __forceinline__ int res_run(const EngineArgs& A, const ResidentLP& lp
 #pragma unroll 4
     for (int q = tid; q < rq; q += kResThreads) {
       rval[q] = __ldcg(gx + rp0 + q);
-      ridx[q] = (uint16_t)ld_ro(I.ri + rp0 + q);
+      ridx[q] = res_index(A, ld_ro(I.ri + rp0 + q), I.n, rb);
     }
 #pragma unroll 4
     for (int q = tid; q < cq; q += kResThreads) {
       cval[q] = __ldcg(gc + cp0 + q);
-      cidx[q] = (uint16_t)ld_ro(I.ci + cp0 + q);
+      cidx[q] = res_index(A, ld_ro(I.ci + cp0 + q), I.m, cb);
     }
-    for (int i = tid; i <= rn; i += kResThreads) rptr[i] = rn ? ld_ro(I.rp + rb + i) - rp0 : 0;
-    for (int i = tid; i <= cn; i += kResThreads) cptr[i] = cn ? ld_ro(I.cp + cb + i) - cp0 : 0;
+    for (int i = tid; i <= rn; i += kResThreads) rptr[i] = res_pointer(A, I.rp + rb, i, rn, rp0, rq, rb);
+    for (int i = tid; i <= cn; i += kResThreads) cptr[i] = res_pointer(A, I.cp + cb, i, cn, cp0, cq, cb);
     for (int i = tid; i < rt1 - rt0; i += kResThreads) {
       const Tile& t = A.rtiles[I.rt_begin + rt0 + i];
       rtile[i] = make_int2(t.begin - rb, t.end - rb);
@@ -503,6 +528,11 @@ __device__ __forceinline__ int res_run(const EngineArgs& A, const ResidentLP& lp
   const int cgrp = threadIdx.x / Lc, csub = threadIdx.x & (Lc - 1), cstep = kResThreads / Lc;
   double sigma = c.eta * c.omega, tau = c.eta / c.omega;
   cluster_sync();          // no peer writes into this CTA before it has loaded
+#ifdef PDLP_BOUNDS_CHECK
+  if (threadIdx.x == 0 && block_flags()[1]) cluster_put(&H.bad, 1, size);
+  cluster_sync();
+  if (H.bad) return -1;
+#endif
 
   while (step < budget && res_hot(c.rmode, c.cmode)) {
     if (c.rmode != R_NONE) {
@@ -710,7 +740,7 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
     const int* src = reinterpret_cast<const int*>(A.inst + lp.inst);
     int* dst = reinterpret_cast<int*>(&H.inst);
     for (int i = threadIdx.x; i < (int)(sizeof(Inst) / sizeof(int)); i += kResThreads) dst[i] = src[i];
-    if (threadIdx.x == 0) H.failed[0] = H.failed[1] = 0;
+    if (threadIdx.x == 0) H.failed[0] = H.failed[1] = H.bad = H.flags[1] = 0;
     __syncthreads();
   }
   const Inst& I = H.inst;
@@ -735,7 +765,9 @@ __global__ void __launch_bounds__(kResThreads, 1) engine_resident(EngineArgs A,
     if (C.rmode == R_NONE && C.cmode == C_NONE) break;           // the LP is done
     if (res_hot(C.rmode, C.cmode)) {
       __syncthreads();                                           // every warp has read C
-      step = res_run<T>(A, lp, S, rank, size, step);
+      const int done = res_run<T>(A, lp, S, rank, size, step);
+      if (done < 0) break;
+      step = done;
       continue;
     }
     // one step of the generic passes
