@@ -203,7 +203,9 @@ typedef struct pdlp_batch_config {
                                    device fault.  2: warps without work in a
                                    pass read their team's state 20 us late
                                    (results must not change).  Either keeps
-                                   every LP on block teams                  */
+                                   every LP on block teams.  3: the second
+                                   on-chip launch of a step reports a failure
+                                   instead of being made                    */
 } pdlp_batch_config;
 
 void pdlp_batch_config_default(pdlp_batch_config* cfg);

@@ -497,7 +497,7 @@ thread_local std::string g_err;
 constexpr size_t kAlign = 256;
 
 // pdlp_batch_config.test_withhold_arrival
-constexpr int kTestWithhold = 1, kTestLateLoads = 2;
+constexpr int kTestWithhold = 1, kTestLateLoads = 2, kTestLaunchFails = 3;
 
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
@@ -870,7 +870,9 @@ static bool res_fits(const Slot& sl, int size) {
 // choose where it runs (a tuning run or the withheld-arrival hook wants the
 // team engine, the infeasibility test short launches).
 static int smallest_cluster(const pdlp_batch* b, const Slot& sl) {
-  if (b->max_cluster < 1 || b->force_set || b->cfg.test_withhold_arrival || sl.detect) return 0;
+  if (b->max_cluster < 1 || b->force_set || sl.detect) return 0;
+  if (b->cfg.test_withhold_arrival == kTestWithhold || b->cfg.test_withhold_arrival == kTestLateLoads)
+    return 0;
   if (sl.m < 1 || sl.n < 1 || sl.m > 65535 || sl.n > 65535) return 0;
   for (const Tile& t : sl.rt) if (t.heavy) return 0;
   for (const Tile& t : sl.ct) if (t.heavy) return 0;
@@ -913,7 +915,8 @@ static void return_on_chip(pdlp_batch* b) {
 // Launches the resident engine for every running slot that has steps left and
 // fits a cluster, each cluster size on a stream of its own; the batch's stream
 // waits for them.  Slots get the smallest cluster that holds them, doubled as
-// long as all of them still fit the device side by side.
+// long as all of them still fit the device side by side.  *count: the LPs of
+// the launches; on failure 0 when nothing has been launched yet.
 static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
   *count = 0;
   if (b->resident.empty()) return PDLP_OK;
@@ -967,7 +970,6 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
       order.push_back(s);
     }
   }
-  *count = (int)order.size();
   if (order.empty()) return PDLP_OK;
   EngineArgs R = A;
   R.team_copies = nullptr;           // the clusters' warps read the State (engine_resident)
@@ -984,7 +986,9 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
       if (!q) PDLP_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
     PDLP_CUDA(cudaEventRecord(b->res_events[5], st));
   }
+  *count = (int)order.size();
   size_t first = 0;
+  int launched = 0;
   for (int k = 4; k >= 0; --k) {
     const size_t n = by_size[k].size();
     if (n == 0) continue;
@@ -994,6 +998,8 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
       const int f32 = b->slots[by_size[k][a]].inst.f32;
       size_t z = a;
       while (z < n && b->slots[by_size[k][z]].inst.f32 == f32) ++z;
+      if (b->cfg.test_withhold_arrival == kTestLaunchFails && launched++ > 0)
+        return fail(PDLP_ERR_CUDA, "engine: a launch on chip failed (test hook)");
       cudaLaunchConfig_t cfg;
       cudaLaunchAttribute attr;
       res_config(1 << k, (int)(z - a), q, &cfg, &attr);
@@ -1416,7 +1422,8 @@ struct Pending {
 static int admit_args(pdlp_batch* b, const pdlp_problem_desc* P, const pdlp_params* params,
                       pdlp_params* prm) {
   if (!b || !P) return fail(PDLP_ERR_ARG, "NULL batch or problem");
-  if (b->broken) return fail(PDLP_ERR_STATE, "batch is unusable after a device wait timed out");
+  if (b->broken)
+    return fail(PDLP_ERR_STATE, "batch is unusable after a device wait timed out or a launch failed");
   pdlp_params_default(prm);
   if (params) *prm = *params;
   const int m = P->m, n = P->n;
@@ -2046,7 +2053,8 @@ int pdlp_batch_admit_many(pdlp_batch* b, int32_t count, const pdlp_problem_desc*
 
 int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
   if (!b) return fail(PDLP_ERR_ARG, "NULL batch");
-  if (b->broken) return fail(PDLP_ERR_STATE, "batch is unusable after a device wait timed out");
+  if (b->broken)
+    return fail(PDLP_ERR_STATE, "batch is unusable after a device wait timed out or a launch failed");
   b->last_ms = 0.0; b->last_bytes = 0.0; b->last_iters = 0;
   if (b->n_running == 0) { if (active_out) *active_out = 0; return PDLP_OK; }
   int rc;
@@ -2115,12 +2123,23 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     PDLP_CUDA(cudaEventRecord(b->ev0, st));
     int n_res = 0;
     if (b->cfg.persistent) {
-      if ((rc = launch_resident(b, A, &n_res))) return rc;
-      if (b->grid > 0) {
+      rc = launch_resident(b, A, &n_res);
+      if (rc == PDLP_OK && b->grid > 0) {
         void* args[] = {&A};
-        PDLP_CUDA(cudaLaunchCooperativeKernel((void*)engine_persistent, dim3(b->grid), dim3(kBlock),
-                                              args, kSmemBytes, st));
-        count_launches(1);
+        const cudaError_t e = cudaLaunchCooperativeKernel((void*)engine_persistent, dim3(b->grid),
+                                                          dim3(kBlock), args, kSmemBytes, st);
+        if (e == cudaSuccess) count_launches(1);
+        else rc = cuda_fail(e, "cudaLaunchCooperativeKernel");
+      }
+      if (rc != PDLP_OK) {
+        // clusters that do run are waited for: they advance their LPs, which
+        // the host then knows nothing of, so the batch ends here
+        if (n_res > 0) {
+          for (cudaStream_t q : b->res_streams) if (q) cudaStreamSynchronize(q);
+          cudaStreamSynchronize(st);
+          b->broken = true;
+        }
+        return rc;
       }
     } else {
       if (b->graph_stale || !b->graph || b->graph_chunk != chunk) {
