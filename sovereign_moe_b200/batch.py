@@ -114,10 +114,12 @@ class BatchEngine:
         shared = []          # device-resident LPs that start from the reference's vector
         for i, prob in enumerate(probs):
             d, k = problem_desc(prob, sync=False)
-            p, kv = params_struct(params, int(prob.A.n), power_start=power_start)
-            if d.memory == _lib.PDLP_MEM_DEVICE and isinstance(power_start, str):
+            if (d.memory == _lib.PDLP_MEM_DEVICE and isinstance(power_start, str)
+                    and power_start == "reference"):
+                p, kv = params_struct(params, int(prob.A.n), power_start=None)
                 shared.append(i)
             else:
+                p, kv = params_struct(params, int(prob.A.n), power_start=power_start)
                 kv = start_with_problem(d, p, kv)
             if hints is not None:
                 p.expected_iterations = float(hints[i])
