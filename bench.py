@@ -17,9 +17,11 @@ value   : solves/s with the LPs already resident in HBM (admission from device
           memory), whole job over all ranks.
 e2e     : the same through the C ABI from pinned host buffers: H2D of every
           LP's arrays, solve, D2H of x, y and reduced costs, inside the timing.
-roofline: the persistent engine kernel; algorithmic bytes of the PDHG
+roofline: the persistent engine kernel alone; algorithmic bytes of the PDHG
           iterations it ran (24 nnz + 4(m+1) + 4(n+1) + 8(10m + 11n) per
-          iteration of an LP, float64) over its CUDA-event time.
+          iteration of an LP, float64) over its CUDA-event time.  LPs stepped
+          on chip read nothing from HBM per iteration; their share of the
+          step is given beside it.
 --impl reference: the CPU restatement of the reference path (oracle/, same
           iterates as sovopt's solve_pdlp bit for bit) on a bounded sample of
           the same LPs, all host threads, rank 0 only.
@@ -46,10 +48,10 @@ METRIC = "LP solves/s at rel KKT 1e-6"
 N_LP = 256
 EPS = 1e-6
 # DRAM bytes per algorithmic byte of engine_persistent on this batch, from one
-# ncu capture of the first 256-step launch of
-# `bench.py --workload engine-steps --iters 300`: dram__bytes_read.sum +
-# dram__bytes_write.sum = 80.43 GB against 75.90 GB of algorithmic bytes.
-TRAFFIC_PER_ALGORITHMIC_BYTE = 80.43 / 75.90
+# ncu capture of its third launch in `bench.py --workload engine-steps --iters
+# 300` (44 steps past the set-up, all 256 LPs on block teams): dram__bytes_read.sum
+# + dram__bytes_write.sum = 15.37 GB against 15.79 GB of algorithmic bytes.
+TRAFFIC_PER_ALGORITHMIC_BYTE = 15.37 / 15.79
 
 
 def load_peaks():
@@ -296,10 +298,12 @@ class GpuArm:
         from sovereign_moe_b200.schedule import IterationModel
         self.model = IterationModel()
         self.latencies = []
-        self.engine_ms = 0.0
-        self.engine_bytes = 0.0
-        self.engine_launches = 0
-        self.engine_kernels = 0
+        self.reset_engines()
+
+    def reset_engines(self):
+        # per engine (block teams, clusters): device ms, algorithmic bytes,
+        # iterations and launches
+        self.engines = [[0.0, 0.0, 0, 0], [0.0, 0.0, 0, 0]]
 
     def step(self, host=False):
         """One batched step: admit every LP, run the batch to completion, fetch
@@ -321,13 +325,10 @@ class GpuArm:
         admit_s = time.perf_counter() - t0
         active = ct.c_int32(1)
         while active.value > 0:
-            k0 = c.pdlp_launch_count()
             L.check(c.pdlp_batch_step(self.eng.h, 1 << 16, ct.byref(active)))
-            self.engine_kernels += c.pdlp_launch_count() - k0
-            ms, by, _ = self.eng.last_timing()
-            self.engine_ms += ms
-            self.engine_bytes += by
-            self.engine_launches += 1
+            for on_chip, total in enumerate(self.engines):
+                for i, v in enumerate(self.eng.last_engine(on_chip)):
+                    total[i] += v
         # every LP's result, x, y and d, and the slots retired, with one
         # synchronisation (pdlp_batch_collect_many)
         n = len(slots)
@@ -449,9 +450,7 @@ def run_gpu(args, rank, world):
     # device-resident timing
     clocks = ClockSampler(local)
     clocks.start()
-    arm.engine_ms = arm.engine_bytes = 0.0
-    arm.engine_launches = 0
-    arm.engine_kernels = 0
+    arm.reset_engines()
     n0 = lib.pdlp_launch_count()
     barrier()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -465,8 +464,7 @@ def run_gpu(args, rank, world):
     dev_ms = ev0.elapsed_time(ev1)
     step_ms = max_over_ranks(dev_ms / args.steps)
     value = N_LP * world / (step_ms / 1000.0)
-    eng_ms, eng_bytes, eng_launches = arm.engine_ms, arm.engine_bytes, arm.engine_launches
-    eng_kernels = arm.engine_kernels
+    (eng_ms, eng_bytes, eng_iters, eng_kernels), chip = [list(e) for e in arm.engines]
 
     # end to end through the C ABI from pinned host buffers (one untimed pass
     # first, so both arms are timed warm)
@@ -566,7 +564,11 @@ def run_gpu(args, rank, world):
                          "algorithmic_bytes_per_launch": (eng_bytes / eng_kernels
                                                           if eng_kernels else None),
                          "kernel": "engine_persistent", "peak_source": peak_kind,
-                         "launches": eng_kernels, "kernel_ms_per_step": eng_ms / args.steps},
+                         "launches": eng_kernels, "kernel_ms_per_step": eng_ms / args.steps,
+                         "iterations_per_step": eng_iters / args.steps,
+                         "on_chip": {"kernel": "engine_resident", "launches": chip[3],
+                                     "ms_per_step": chip[0] / args.steps,
+                                     "iterations_per_step": chip[2] / args.steps}},
             "cpu_baseline": cpu,
             "clocks": clk,
             "gpu_launches": int(launches),
@@ -672,10 +674,14 @@ def run_engine_steps(args):
         while done < args.iters:
             n = min(256, args.iters - done)
             active = eng.step(n)
-            ms, by, its = eng.last_timing()
-            launches.append({"steps": n, "active_after": active, "ms": ms,
-                             "us_per_step": 1000.0 * ms / n, "iterations": its,
-                             "achieved_GBps": by / ms / 1e6 if ms else 0.0})
+            ms, _, its = eng.last_timing()
+            tms, tby, tits, tk = eng.last_engine(False)
+            cms, _, cits, ck = eng.last_engine(True)
+            launches.append({"steps": n, "active_after": active, "ms": ms, "iterations": its,
+                             "teams": {"launches": tk, "ms": tms, "iterations": tits,
+                                       "algorithmic_bytes": tby,
+                                       "achieved_GBps": tby / tms / 1e6 if tms else 0.0},
+                             "on_chip": {"launches": ck, "ms": cms, "iterations": cits}})
             done += n
             if active == 0:
                 break

@@ -275,10 +275,15 @@ int pdlp_batch_scaling(pdlp_batch* b, int32_t slot, double* row_scale, double* c
                        double* obj_scale, int32_t memory);
 /* Device bytes a slot for this problem would take (admission planning). */
 int64_t pdlp_slot_bytes(int32_t m, int32_t n, int64_t nnz);
-/* Per-kernel timing of the last pdlp_batch_step: total device milliseconds
- * and algorithmic bytes moved by the PDHG iterations. */
+/* The last pdlp_batch_step: total device milliseconds and algorithmic bytes
+ * of the PDHG iterations. */
 int pdlp_batch_last_timing(pdlp_batch* b, double* ms, double* iter_bytes,
                            int64_t* iterations);
+/* The share of it of the clusters (on_chip != 0) or of the block teams; the two
+ * run one after the other.  The algorithmic bytes of an iteration on chip are
+ * not traffic: its matrix and vectors are in shared memory. */
+int pdlp_batch_last_engine(pdlp_batch* b, int32_t on_chip, double* ms, double* iter_bytes,
+                           int64_t* iterations, int64_t* launches);
 
 /* ---- engine autotuner --------------------------------------------------- *
  * No counterpart in the reference, whose kernels have one fixed launch shape

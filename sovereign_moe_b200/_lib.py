@@ -161,6 +161,8 @@ SIGNATURES = {
     "pdlp_slot_bytes": ([_i32, _i32, _i64], ctypes.c_int64),
     "pdlp_batch_last_timing": ([_c_p, ctypes.POINTER(_d), ctypes.POINTER(_d),
                                 ctypes.POINTER(_i64)], ctypes.c_int),
+    "pdlp_batch_last_engine": ([_c_p, _i32, ctypes.POINTER(_d), ctypes.POINTER(_d),
+                                ctypes.POINTER(_i64), ctypes.POINTER(_i64)], ctypes.c_int),
     "pdlp_spmv_f64": ([_i32, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p], ctypes.c_int),
     "pdlp_spmv_f32": ([_i32, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p], ctypes.c_int),
     "pdlp_spmv_ex_f64": ([_i32, _i32, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p], ctypes.c_int),

@@ -206,6 +206,17 @@ class BatchEngine:
                                                    ctypes.byref(it)))
         return ms.value, by.value, it.value
 
+    def last_engine(self, on_chip):
+        """The last step's share of one engine, the clusters (``on_chip``) or the
+        block teams: (device ms, algorithmic PDHG bytes, PDHG iterations,
+        launches).  On chip an iteration reads nothing from HBM."""
+        ms, by = ctypes.c_double(), ctypes.c_double()
+        it, launches = ctypes.c_int64(), ctypes.c_int64()
+        _lib.check(self.lib.pdlp_batch_last_engine(self.h, 1 if on_chip else 0, ctypes.byref(ms),
+                                                   ctypes.byref(by), ctypes.byref(it),
+                                                   ctypes.byref(launches)))
+        return ms.value, by.value, it.value, launches.value
+
     def slot_bytes(self, m, n, nnz):
         return int(self.lib.pdlp_slot_bytes(int(m), int(n), int(nnz)))
 

@@ -625,6 +625,10 @@ struct pdlp_batch {
   bool graph_stale = true;
   double last_ms = 0.0, last_bytes = 0.0;
   long long last_iters = 0;
+  struct EngineWork {                  // of the last step, by engine: block teams, clusters
+    double ms = 0.0, bytes = 0.0;
+    long long iters = 0, launches = 0;
+  } last_engine[2];
   std::vector<long long> iters_before;
   std::vector<long long> steps_left;   // per slot: steps it may still run in this call
   size_t bytes_pending = 0;            // arenas of admissions in progress
@@ -652,7 +656,8 @@ struct pdlp_batch {
   int* h_res_steps = nullptr;          // pinned / device: steps each one ran
   int* d_res_steps = nullptr;
   cudaStream_t res_streams[5] = {};    // one per cluster size
-  cudaEvent_t res_events[6] = {};      // ready, then one per cluster size
+  cudaEvent_t res_events[6] = {};      // one per cluster size, then ready
+  cudaEvent_t res_done = nullptr;      // the launch's clusters have finished
 };
 
 namespace pdlp {
@@ -1007,6 +1012,7 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
                                    (const ResidentLP*)(b->d_res + first + a),
                                    b->d_res_steps + first + a));
       count_launches(1);
+      b->last_engine[1].launches += 1;
       a = z;
     }
     if (sizes > 1) {
@@ -1983,6 +1989,7 @@ int pdlp_batch_create(const pdlp_batch_config* cfg, void* stream, pdlp_batch** o
   cudaMemcpyAsync(b->d_inst, zero.data(), sizeof(Inst) * zero.size(), cudaMemcpyHostToDevice, b->stream);
   cudaEventCreate(&b->ev0);
   cudaEventCreate(&b->ev1);
+  cudaEventCreate(&b->res_done);
   if (!b->cfg.persistent &&
       (e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking)) != cudaSuccess)
     return bail(e, "cudaStreamCreateWithFlags");
@@ -2022,6 +2029,7 @@ int pdlp_batch_destroy(pdlp_batch* b) {
   cudaFree(b->d_res_steps);
   for (cudaStream_t q : b->res_streams) if (q) cudaStreamDestroy(q);
   for (cudaEvent_t q : b->res_events) if (q) cudaEventDestroy(q);
+  if (b->res_done) cudaEventDestroy(b->res_done);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   delete b;
@@ -2056,6 +2064,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
   if (b->broken)
     return fail(PDLP_ERR_STATE, "batch is unusable after a device wait timed out or a launch failed");
   b->last_ms = 0.0; b->last_bytes = 0.0; b->last_iters = 0;
+  b->last_engine[0] = b->last_engine[1] = {};
   if (b->n_running == 0) { if (active_out) *active_out = 0; return PDLP_OK; }
   int rc;
   cudaStream_t st = b->stream;
@@ -2124,11 +2133,15 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     int n_res = 0;
     if (b->cfg.persistent) {
       rc = launch_resident(b, A, &n_res);
+      if (rc == PDLP_OK && n_res > 0 && b->grid > 0) {
+        const cudaError_t e = cudaEventRecord(b->res_done, st);
+        if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventRecord");
+      }
       if (rc == PDLP_OK && b->grid > 0) {
         void* args[] = {&A};
         const cudaError_t e = cudaLaunchCooperativeKernel((void*)engine_persistent, dim3(b->grid),
                                                           dim3(kBlock), args, kSmemBytes, st);
-        if (e == cudaSuccess) count_launches(1);
+        if (e == cudaSuccess) { count_launches(1); b->last_engine[0].launches += 1; }
         else rc = cuda_fail(e, "cudaLaunchCooperativeKernel");
       }
       if (rc != PDLP_OK) {
@@ -2166,6 +2179,7 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
       }
       PDLP_CUDA(cudaGraphLaunch(b->graph, st));
       count_launches(2 * chunk);
+      b->last_engine[0].launches += 2 * chunk;
     }
     PDLP_CUDA(cudaEventRecord(b->ev1, st));
     PDLP_CUDA(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, st));
@@ -2178,6 +2192,11 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, b->ev0, b->ev1);
     total_ms += ms;
+    // clusters first, then block teams
+    float chip_ms = n_res > 0 ? ms : 0.f;
+    if (n_res > 0 && b->grid > 0) cudaEventElapsedTime(&chip_ms, b->ev0, b->res_done);
+    b->last_engine[1].ms += chip_ms;
+    b->last_engine[0].ms += ms - chip_ms;
 #ifdef PDLP_TRACE
     {
       long long h[1280];
@@ -2235,6 +2254,8 @@ int pdlp_batch_step(pdlp_batch* b, int64_t max_steps, int32_t* active_out) {
       b->iters_before[s] = hs.iters_done;
       b->last_iters += d;
       b->last_bytes += d * sl.bytes_per_iter;
+      b->last_engine[sl.on_chip()].iters += d;
+      b->last_engine[sl.on_chip()].bytes += d * sl.bytes_per_iter;
       if (hs.status != PDLP_STATUS_RUNNING) { sl.running = false; b->dirty = true; }
       else {
         ++running;
@@ -2277,6 +2298,17 @@ int pdlp_batch_last_timing(pdlp_batch* b, double* ms, double* iter_bytes, int64_
   if (ms) *ms = b->last_ms;
   if (iter_bytes) *iter_bytes = b->last_bytes;
   if (iterations) *iterations = b->last_iters;
+  return PDLP_OK;
+}
+
+int pdlp_batch_last_engine(pdlp_batch* b, int32_t on_chip, double* ms, double* iter_bytes,
+                           int64_t* iterations, int64_t* launches) {
+  if (!b) return fail(PDLP_ERR_ARG, "NULL batch");
+  const auto& w = b->last_engine[on_chip != 0];
+  if (ms) *ms = w.ms;
+  if (iter_bytes) *iter_bytes = w.bytes;
+  if (iterations) *iterations = w.iters;
+  if (launches) *launches = w.launches;
   return PDLP_OK;
 }
 
