@@ -115,14 +115,18 @@ __device__ __forceinline__ void team_read(const EngineArgs& A, WarpSmem& W, int 
 __device__ __forceinline__ void team_publish(const EngineArgs& A, const WarpSmem& W, const State* S) {
   if (A.team_copies == nullptr) return;
   TeamCopy* o = A.team_copies + 2 * (size_t)W.inst_id + ((W.pass + 1u) & 1u);
-  o->eta = S->eta;
-  o->omega = S->omega;
-  o->k = S->k;
-  o->rmode = S->rmode;
-  o->cmode = S->cmode;
-  o->cprimal = S->cprimal;
-  o->xcommit = S->xcommit;
-  o->ycommit = S->ycommit;
+  const double eta = S->eta, omega = S->omega;
+  const long long k = S->k;
+  const int rmode = S->rmode, cmode = S->cmode, cprimal = S->cprimal;
+  const int xcommit = S->xcommit, ycommit = S->ycommit;
+  o->eta = eta;
+  o->omega = omega;
+  o->k = k;
+  o->rmode = rmode;
+  o->cmode = cmode;
+  o->cprimal = cprimal;
+  o->xcommit = xcommit;
+  o->ycommit = ycommit;
 }
 
 // Writes down what the copy is ahead of the state: its normal iterations, one
