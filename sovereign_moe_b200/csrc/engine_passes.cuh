@@ -197,19 +197,17 @@ __device__ __forceinline__ bool warp_finish(const EngineArgs& A, const Tile& t, 
   if (!last) return false;
   __syncwarp();                            // order the lanes' reads after lane 0's acquire
   double v[kNP];
-  if (need_red) {
 #pragma unroll
-    for (int s = 0; s < kNP; ++s) v[s] = identity_of(ops.op(s));
-    for (int tt = gt.x + lane; tt < gt.y; tt += 32) {
+  for (int s = 0; s < kNP; ++s) v[s] = identity_of(ops.op(s));
+  for (int tt = gt.x + lane; tt < gt.y; tt += 32) {
 #pragma unroll
-      for (int s = 0; s < kNP; ++s)
-        if (s < slots) v[s] = combine(v[s], ld_mut(tp + (size_t)tt * kNP + s), ops.op(s));
-    }
-    warp_reduce(v, ops, slots);
-    if (lane == 0 && g_last - g_first > 1) {
+    for (int s = 0; s < kNP; ++s)
+      if (s < slots) v[s] = combine(v[s], ld_mut(tp + (size_t)tt * kNP + s), ops.op(s));
+  }
+  warp_reduce(v, ops, slots);
+  if (lane == 0 && g_last - g_first > 1) {
 #pragma unroll
-      for (int s = 0; s < kNP; ++s) A.gpartials[(size_t)g * kNP + s] = v[s];
-    }
+    for (int s = 0; s < kNP; ++s) A.gpartials[(size_t)g * kNP + s] = v[s];
   }
   __syncwarp();
   if (g_last - g_first == 1) {
@@ -227,18 +225,16 @@ __device__ __forceinline__ bool warp_finish(const EngineArgs& A, const Tile& t, 
   last = __shfl_sync(kFull, last, 0);
   if (!last) return false;
   __syncwarp();
-  if (need_red) {
 #pragma unroll
-    for (int s = 0; s < kNP; ++s) v[s] = identity_of(ops.op(s));
-    for (int gg = g_first + lane; gg < g_last; gg += 32) {
+  for (int s = 0; s < kNP; ++s) v[s] = identity_of(ops.op(s));
+  for (int gg = g_first + lane; gg < g_last; gg += 32) {
 #pragma unroll
-      for (int s = 0; s < kNP; ++s)
-        if (s < slots) v[s] = combine(v[s], ld_mut(A.gpartials + (size_t)gg * kNP + s), ops.op(s));
-    }
-    warp_reduce(v, ops, slots);
-#pragma unroll
-    for (int s = 0; s < kNP; ++s) res[s] = v[s];
+    for (int s = 0; s < kNP; ++s)
+      if (s < slots) v[s] = combine(v[s], ld_mut(A.gpartials + (size_t)gg * kNP + s), ops.op(s));
   }
+  warp_reduce(v, ops, slots);
+#pragma unroll
+  for (int s = 0; s < kNP; ++s) res[s] = v[s];
   if (lane == 0) A.counters[2 * t.inst + side] = 0;
   return true;
 }

@@ -369,16 +369,16 @@ int long_row_list(cudaStream_t st, size_t entries, int** out) {
 // Rows per warp of the streamed pass, 4 to 32: as many as leave
 // kSpmvTargetWarps warps (56 of an SM's 64).  A warp walks its rows' runs of
 // 256 entries one after another, so few long rows want few rows a warp, and
-// many rows want many, to fill the runs.  Float64 on B200, us per product with
-// 4 / 8 / 16 / 32 rows a warp: 50,000 rows of 39 entries 17 / 19 / 28 / 44; 100,000
-// of 15: 17.4 / 13.9 / 14.6 / 16.4; 200,000 of 15: 35 / 26.4 / 25.2 / 26.0; 300,000 of
-// 6: 33 / 20.8 / 16.1 / 15.1; 600,000 of 5: 65 / 38 / 27 / 22.1; 3,000,000 of 3: 311 /
-// 166 / 98 / 69.  64 rows a warp (two per lane) gained on uniform rows of 3
-// entries (58) and lost on power-law ones (float32 101 against 97) and on
-// 200,000 rows of 15 (40).  Each row's sum is the same whichever warp takes
-// it.  Six blocks per SM pay in float64 (40 registers: 74.4 and 99.5 us on the
-// power law's two products, 82.2 and 101.1 without the bound) and lose in
-// float32 (71.5 and 93.8 against 65.4 and 89.8).
+// many rows want many, to fill the runs.  Float64 on B200, us per product in a
+// stream of products with 4 / 8 / 16 / 32 rows a warp: 50,000 rows of 39 entries
+// 16.7 / 18.2 / 28.4 / 49; 100,000 of 15: 17.3 / 15.2 / 14.3 / 22.2; 200,000 of 15:
+// 29 / 22.2 / 22.3 / 22.6; 300,000 of 6: 33 / 20.8 / 17.0 / 15.3; 600,000 of 5: 57 / 32 /
+// 22.2 / 18.5; 3,000,000 of 3: 289 / 154 / 92 / 64.  64 rows a warp (two per lane)
+// gained on uniform rows of 3 entries and lost on power-law ones and on 200,000
+// rows of 15.  Each row's sum is the same whichever warp takes it.  Six blocks
+// per SM pay in float64 (40 registers: 71.8 and 99.9 us on the power law's two
+// products, 79.9 and 101.5 without the bound) and lose in float32 (68.7 and 92.1
+// against 62.7 and 82.6).
 constexpr int kSpmvTargetWarps = 148 * 56;
 constexpr int kLongBlocks = 592;
 int rows_per_warp(int m) {
