@@ -99,8 +99,10 @@ __device__ void late_load() {
 // A team of one LP (team_inst) keeps the LP's scheduling fields in its warps
 // (TeamCopy); they start from the State, which no pass may change before every
 // warp has read it, hence a barrier before the first step.  Its normal iterations then cost two barriers and nothing else:
-// no counters, no finisher, no state read.  Alone, in us per iteration with
-// checks and set-up: a 3 x 5 LP 16.2 -> 13.0, 230 x 2,025 20.4 -> 17.9.
+// no counters, no finisher, no state read.  Alone in this engine, in us per
+// iteration with checks and set-up, before the copies (and the stop bit, the
+// one-group reduction and a block per two tiles, which came with them) and now:
+// a 3 x 5 LP 16.2 / 11.2, 230 x 2,025 20.4 / 17.6, 10,000 x 40,000 in float32 28.8 / 22.0.
 __global__ void __launch_bounds__(kBlock, 4) engine_persistent(EngineArgs A) {
   WarpSmem* ws = block_warps();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -889,7 +891,7 @@ static int smallest_cluster(const pdlp_batch* b, const Slot& sl) {
 // The most blocks an instance can use: a warp's tile gathers 512 scattered
 // doubles, and the warps of an SM share its load units, so two tiles a block
 // on twice the SMs finish a pass sooner than one per warp (10,000 x 40,000 in
-// float32 alone, us per iteration: four tiles a block 28.2, two 22.3, one 23.6 --
+// float32 alone, us per iteration when it was chosen: four tiles a block 28.2, two 22.3, one 23.6 --
 // more blocks also mean more arrivals at the barriers; 35 LPs of up to 1,500
 // rows: 111, 98 and 96 ms).
 constexpr int kTilesPerBlock = 2;
@@ -900,9 +902,10 @@ constexpr int kTilesPerBlock = 2;
 // goes on there beside them (both engines give the same bits), until only LPs
 // that fit clusters are left; so a long solve on chip holds nobody up.
 // (It moves only to a team of its own: a team of several LPs steps all of them
-// by one budget.)  256 uneven LPs, a fifth of them too large for a cluster: LPs/s with estimates,
-// ms without, by the steps before an LP moves: 128 550, 442; 256 546, 443; 512
-// 540, 447; 1,024 535, 450; 2,048 530, 456; 4,096 513, 456; 16,384 498, 484.
+// by one budget.)  256 uneven LPs, a fifth of them too large for a cluster, when
+// the limit was chosen: LPs/s with estimates, ms without, by the steps before an
+// LP moves: 128 550, 442; 256 546, 443; 512 540, 447; 1,024 535, 450; 2,048 530,
+// 456; 4,096 513, 456; 16,384 498, 484.
 // Alone the limit lets LPs that do not all fit the GPU at once take turns too.
 constexpr int kResSteps = 16384, kResStepsBeside = 256;
 
@@ -930,8 +933,8 @@ static int launch_resident(pdlp_batch* b, const EngineArgs& A, int* count) {
   if (!b->h_res_steps) PDLP_CUDA(cudaMallocHost((void**)&b->h_res_steps, sizeof(int) * slots));
   if (!b->d_res) PDLP_CUDA(cudaMalloc((void**)&b->d_res, sizeof(ResidentLP) * slots));
   if (!b->d_res_steps) PDLP_CUDA(cudaMalloc((void**)&b->d_res_steps, sizeof(int) * slots));
-  // growing stops at 8 SMs: 16 gained nothing on LPs that fit 2 (230 x 2,025: 8.6
-  // us per iteration on 4 SMs, 8.4 on 8, 8.3 on 16)
+  // growing stops at 8 SMs: 16 gained nothing on LPs that fit 2 (230 x 2,025 to its
+  // tolerance, us per iteration: 7.9 on 4 SMs, 6.9 on 8, 6.9 on 16)
   constexpr int kGrowTo = 8;
   long long sms = 0;
   for (int s : b->resident) sms += b->slots[s].cluster;

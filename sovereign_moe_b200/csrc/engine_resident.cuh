@@ -21,14 +21,14 @@
 // loads the resident data from the arena (9 us) and writes the vectors back.
 //
 // Measured on B200, alone, us per iteration with set-up and checks, team engine
-// against this one: 3 x 5 11.9 / 5.2, 230 x 2,025 17.6 / 7.3; 347 x 2,776 solved by
-// solve_pdlp for 1,024 iterations 21.4 -> 6.5 ms.  An iteration of 230 x 2,025 on
-// eight SMs takes 7,500 cycles: 1,200 products (bound by bank conflicts of the
-// scattered 8-byte reads), 3,300 row sums and steps (a chain of dependent
-// float64 adds and a division per row), 1,600 barriers with the remote stores
-// they wait for, 950 the line search's share; a generic step takes 25 us, about
-// 54 of them in a solve of 448 iterations.  At 16 SMs the products shrink and
-// nothing else does.
+// against this one: 3 x 5 (704 iterations) 11.2 / 4.4, 230 x 2,025 (448) 17.6 / 6.9,
+// 347 x 2,776 (1,024) 16.7 / 6.6.  By clock stamps of an earlier build of the same
+// loop an iteration of 230 x 2,025 on eight SMs takes 7,500 cycles: 1,200 products
+// (bound by bank conflicts of the scattered 8-byte reads), 3,300 row sums and
+// steps (a chain of dependent float64 adds and a division per row), 1,600
+// barriers with the remote stores they wait for, 950 the line search's share; a
+// generic step takes about 20 us, and a solve of 448 iterations has about 54 of
+// them.  At 16 SMs the products shrink and nothing else does.
 //
 // Row sums, element-wise steps, tile partials and reduction trees are those of
 // engine_passes.cuh, operand for operand, so every LP's bits are the same in

@@ -7,6 +7,7 @@ overwrites one entry of an admitted LP, with values that stay inside the slot's
 memory.  Skipped with a product build, which has neither."""
 
 import ctypes
+import os
 
 import numpy as np
 import pytest
@@ -16,6 +17,10 @@ from sovereign_moe_b200.batch import BatchEngine
 from sovereign_moe_b200.pdlp import PDLPParams
 
 pytestmark = pytest.mark.gpu
+
+DEFINES = _lib.LIB_PATH + ".defines"          # what the library was built with
+if not (os.path.exists(DEFINES) and "PDLP_BOUNDS_CHECK" in open(DEFINES).read()):
+    pytest.skip("not a bounds-checked build", allow_module_level=True)
 
 LATE = 2          # the test hook that keeps every LP on block teams
 
@@ -31,8 +36,6 @@ def _lp(m, n, per_col):
 @pytest.mark.parametrize("which", ["row index", "column index", "row pointer", "column pointer"])
 @pytest.mark.parametrize("shape", [(63, 65, 5), (900, 4500, 9)])
 def test_a_bad_entry_ends_the_step_with_an_error(shape, which, precision, hook):
-    if not hasattr(_lib.load(), "pdlp_batch_test_overwrite"):
-        pytest.skip("not a bounds-checked build")
     m, n, _ = shape
     prob = _lp(*shape)
     nnz = int(prob.A.nnz)
